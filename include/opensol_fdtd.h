@@ -103,8 +103,8 @@ int os_fdtd2d_read_cb(OsFdtd2D *h, float *cb);
  * rows per CTA, 0 = chosen per grid, and a border kernel over the rest) or 0 (one H_z and one E kernel per step) with
  * steps_per_launch 1 or 2: with 2, on a grid without conductivity or magnetic cells whose rows are a multiple of 4
  * cells, the interior box advances two steps per launch and the border two single steps through a scratch field set
- * (allocated by this call), except where the next step is a DFT sample step or field probes are set; results are
- * bit-identical either way.  The E_z-only calls (set_materials,
+ * (allocated by this call), except where the next step is a DFT sample step or field probes are set; variant 3 is
+ * automatic as for E_z engines; results are bit-identical either way.  The E_z-only calls (set_materials,
  * set_coefficients, read_cb, autotune, plan_info, batch, adjoint) return OS_ERR_STATE on an H_z handle and the
  * H_z-only calls below on an E_z handle.
  * ---------------------------------------------------------------------------------------------------------------- */
@@ -244,7 +244,10 @@ int os_fdtd2d_advance_noalloc(OsFdtd2D *h, int64_t n_steps, const float *line_va
  * double-buffered kernels, tile_rows rows per interior tile (0, the default: chosen from the grid so that the tiles
  * fill the device's warp slots once, 8..128 rows) and the frame around the interior advanced one step per launch;
  * variant 2 the same with the blocked general kernel on the frame; variant 0 launches one H and one E kernel per
- * step.
+ * step; variant 3 (what the Python engines ask for) is automatic: where the grid fits the chip (about 2 M cells), a
+ * whole chunk of steps runs in one cooperative launch with the fields in registers, whatever sources, poles, plane-wave
+ * boxes, maps and probes the engine has; elsewhere, under stream capture, with profiling on and in
+ * os_fdtd2d_advance_noalloc, variant 1 runs.
  * Every choice gives bit-identical results.  No open_sol counterpart (open_sol launches per half step). */
 int os_fdtd2d_configure(OsFdtd2D *h, int32_t variant, int32_t steps_per_launch, int32_t tile_rows);
 

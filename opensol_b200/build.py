@@ -20,7 +20,8 @@ CSRC = os.path.join(HERE, 'csrc')
 LIB_DIR = os.path.join(HERE, '_lib')
 OBJ_DIR = os.path.join(LIB_DIR, 'obj')
 LIB_NAME = 'libopensol_fdtd.so'
-SOURCES = ['common.cu', 'fdtd2d.cu', 'fdtd3d.cu']
+SOURCES = ['common.cu', 'fdtd2d.cu', 'fdtd2d_resident.cu', 'fdtd2d_resident_ez_plain.cu', 'fdtd2d_resident_ez_gen.cu',
+           'fdtd2d_resident_hz_plain.cu', 'fdtd2d_resident_hz_gen.cu', 'fdtd3d.cu']
 ARCH = ['-gencode', 'arch=compute_100a,code=sm_100a']
 FLAGS = ['-O3', '-lineinfo', '-std=c++17', '-fmad=false', '-Xcompiler', '-fPIC', '-Xcompiler', '-O2']
 _INCLUDE = re.compile(r'^\s*#include\s+"([^"]+)"', re.M)

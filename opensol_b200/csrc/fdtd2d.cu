@@ -18,6 +18,7 @@
 #include "fdtd2d_hz.cuh"
 #include "fdtd2d_hz2.cuh"
 #include "fdtd2d_frame.cuh"
+#include "fdtd2d_resident.cuh"
 
 #include <algorithm>
 
@@ -94,6 +95,7 @@ struct OsFdtd2D {
     bool cpml_set[4] = {false, false, false, false};
     std::vector<float> host_inv[4];       // inv_dx_e, inv_dx_h, inv_dy_e, inv_dy_h (host copies: interior check)
     int32_t variant = 1;                  // 0: per-half-step kernels, 1: temporally blocked
+    bool automatic = false;               // the resident form where it fits, else `variant`
     int32_t steps_per_launch = 3;         // T of the blocked kernels
     int32_t tile_rows = 0;                // rows per interior tile (0: chosen from the grid, interior_rows)
     int32_t gen_tile_rows = 16;           // rows per general tile
@@ -132,6 +134,14 @@ struct OsFdtd2D {
     float dt_hz = 0.0f, eps0_hz = 0.0f;   // dt and eps0 of the lossless form
     int32_t hz_rows = 0;                  // rows per CTA of the fused step kernel (0: chosen per grid)
     int sm_count = 148;                   // multiprocessors of the device (launch sizing)
+    // resident form (fdtd2d_resident_kernel.cuh): the strips' first rows, the boundary rows in flight and their number, the
+    // flux lines' samples of a chunk
+    std::vector<int32_t> res_rows;        // host copy of the strips' first rows (empty: not planned)
+    os::DeviceArray<int32_t> res_row_start;
+    os::DeviceArray<uint64_t> res_mail;
+    os::DeviceArray<float> res_stage;
+    int32_t res_smem_limit = 0;           // shared memory a block may have
+    uint32_t res_epoch = 1;
 };
 
 namespace os {
@@ -347,6 +357,7 @@ extern "C" int os_fdtd2d_destroy(OsFdtd2D *h) {
         give(h->jz_total);
         give(h->probe_rows), give(h->probe_stage);
         give(h->err), give(h->line_values), give(h->phases);
+        give(h->res_row_start), give(h->res_mail), give(h->res_stage);
         pool_events_done(ev);
     }
     for (cudaEvent_t e : h->prof_events) cudaEventDestroy(e);
@@ -1795,6 +1806,214 @@ static int advance_hz(OsFdtd2D *h, int64_t n_steps, int64_t first_sample, int64_
     return OS_OK;
 }
 
+// ---- resident form (fdtd2d_resident_kernel.cuh): the whole chunk in one cooperative launch, fields in registers
+
+// Strips of rows of the resident form, one per multiprocessor: first rows of each and the end.  An x-side CPML row
+// costs about one and a half plain rows (two more psi updates), so the strips are cut by that weight.
+static std::vector<int32_t> resident_strips(const OsFdtd2D *h) {
+    const OsGrid2D &g = h->grid;
+    const int n = std::min(h->sm_count, g.nx);
+    std::vector<double> sum(g.nx + 1, 0.0);
+    for (int i = 0; i < g.nx; ++i) {
+        const bool layer = ((g.cpml_sides & 1) && i <= g.npml) || ((g.cpml_sides & 2) && i >= g.nx - g.npml - 1);
+        sum[i + 1] = sum[i] + (layer ? 1.5 : 1.0);
+    }
+    std::vector<int32_t> first(n + 1, 0);
+    for (int c = 1; c <= n; ++c) {
+        const double want = sum[g.nx] * c / n;
+        int i = first[c - 1] + 1;
+        while (i < g.nx - (n - c) && sum[i] + 0.5 * (sum[i + 1] - sum[i]) < want) ++i;
+        first[c] = c == n ? g.nx : i;
+    }
+    return first;
+}
+
+static Res2DJob resident_job(const OsFdtd2D *h) {
+    Res2DJob p{};
+    const OsGrid2D &g = h->grid;
+    const int c = h->cur;
+    p.hz = h->polarization;
+    p.nx = g.nx, p.ny = g.ny, p.px = g.periodic_x, p.py = g.periodic_y, p.npml = g.npml;
+    p.n_cta = (int32_t)h->res_rows.size() - 1;
+    p.f = h->ez[c].ptr, p.a = h->hx[c].ptr, p.b = h->hy[c].ptr;
+    p.ca = h->has_ca ? h->ca.ptr : nullptr;
+    p.cb = h->cb.ptr;
+    p.ca_y = h->has_ca ? h->ca_y.ptr : nullptr;
+    p.cb_y = h->cb_y.ptr;
+    p.da = h->has_dadb ? h->da.ptr : nullptr;
+    p.db = h->has_dadb ? h->db.ptr : nullptr;
+    p.da_u = h->da_uniform, p.db_u = h->db_uniform;
+    p.inv_dx_e = h->inv_dx_e.ptr, p.inv_dx_h = h->inv_dx_h.ptr;
+    p.inv_dy_e = h->inv_dy_e.ptr, p.inv_dy_h = h->inv_dy_h.ptr;
+    for (int s = 0; s < 4; ++s) {
+        if (!(g.cpml_sides & (1 << s))) continue;
+        p.cpml_mask |= 1 << s;
+        p.cpml_rows[s] = h->cpml_rows[s].ptr;
+        p.psi_e[s] = h->psi_e[c][s].ptr;
+        p.psi_h[s] = h->psi_h[c][s].ptr;
+    }
+    p.m = h->sample_interval;
+    p.n_lines = (int32_t)h->lines.size();
+    for (int l = 0; l < p.n_lines; ++l) {
+        const LineSource2D &L = *h->lines[l];
+        p.lines[l] = ResLine{L.axis, L.position, L.lo, L.hi, L.profile.ptr};
+    }
+    p.n_probes = h->probes.n;
+    for (int k = 0; k < h->probes.n; ++k)
+        p.probes[k] = ResProbe{h->probes.ix[k], h->probes.iy[k], h->probes.comp[k], 0,
+                               h->probe_rows.ptr + (size_t)k * h->probe_capacity, h->probes.start[k]};
+    p.n_poles = (int32_t)h->poles.size();
+    for (int kind = 0, k = 0; kind < 2; ++kind)
+        for (auto &q : h->poles) {
+            if (q->kind != kind) continue;
+            p.poles[k++] = ResPole{q->kind, q->comp, q->i0, q->i1, q->j0, q->j1, q->damping, q->restoring, q->drive.ptr,
+                                   q->a.ptr, q->b.ptr};
+            p.n_drude += kind == 0;
+        }
+    p.inv_dt = h->inv_dt;
+    p.n_maps = (int32_t)h->maps.size();
+    for (int k = 0; k < p.n_maps; ++k) {
+        const DftMap2D &d = *h->maps[k];
+        p.maps[k] = ResMap{d.x0, d.y0, d.ds, d.mx, d.my, d.nf, nullptr, nullptr, d.acc.ptr};
+    }
+    p.n_tfsf = (int32_t)h->tfsf.size();
+    for (int k = 0; k < p.n_tfsf; ++k) {
+        const Tfsf2D &t = *h->tfsf[k];
+        ResTfsf &q = p.tfsf[k];
+        q.x0 = t.x0, q.x1 = t.x1, q.y0 = t.y0, q.y1 = t.y1, q.aux_x0 = t.aux_x0, q.aux_n = t.aux_n;
+        q.source_index = t.source_index;
+        for (int e = 0; e < 4; ++e) q.coef_h[e] = t.coef_h[e], q.coef_e[e] = t.coef_e[e];
+        q.mur_lo = t.mur_lo, q.mur_hi = t.mur_hi;
+        q.aux_e = t.aux_ez.ptr, q.aux_h = t.aux_hy.ptr;
+        q.aux_coef_h = t.aux_coef_h.ptr, q.aux_coef_e = t.aux_coef_e.ptr;
+    }
+    p.err = h->err.ptr;
+    p.stall_probe_ns = h->stall_probe_ns;
+    return p;
+}
+
+// Whether the handle's chunks run in the resident form now (job, shape and smem filled), planning its strips on the
+// first call.  It takes every feature of the per-step kernels within the parameter block's limits, on any grid whose
+// strips fit a kernel shape (registers: about 2 M cells) and a multiprocessor's shared memory; stream capture keeps the
+// launch-per-step forms, whose work a captured graph may replay beside other kernels.
+static int resident_applies(OsFdtd2D *h, Res2DJob &job, int *shape, size_t *smem, bool *yes) {
+    *yes = false;
+    const OsGrid2D &g = h->grid;
+    if (!h->automatic || h->profiling || g.nx < 2 || g.ny < 2) return OS_OK;
+    if (h->lines.size() > RES_MAX_LINES || h->fluxes.size() > RES_MAX_MONS || h->maps.size() > RES_MAX_MAPS ||
+        h->poles.size() > RES_MAX_POLES || h->tfsf.size() > RES_MAX_TFSF)
+        return OS_OK;
+    if (res2d_shape(g.ny, (g.nx + h->sm_count - 1) / h->sm_count) < 0) return OS_OK;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    OS_CUDA(cudaStreamIsCapturing(h->stream, &capture));
+    if (capture != cudaStreamCaptureStatusNone) return OS_OK;
+    if (h->res_rows.empty()) {
+        h->res_rows = resident_strips(h);
+        OS_CUDA(cudaDeviceGetAttribute(&h->res_smem_limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
+        h->res_smem_limit -= 1024;   // the kernel's own static shared memory
+    }
+    int max_rows = 0;
+    for (size_t c = 0; c + 1 < h->res_rows.size(); ++c)
+        max_rows = std::max(max_rows, h->res_rows[c + 1] - h->res_rows[c]);
+    *shape = res2d_shape(g.ny, max_rows);
+    if (*shape < 0) return OS_OK;
+    job = resident_job(h);
+    const bool lo = g.cpml_sides & 1, hi = g.cpml_sides & 2;
+    auto rows_in = [](int a, int b, int c, int d) { return std::max(0, std::min(b, d) - std::max(a, c)); };
+    *smem = 0;
+    for (size_t c = 0; c + 1 < h->res_rows.size(); ++c) {
+        const int a = h->res_rows[c], b = h->res_rows[c + 1];
+        const int upper = hi ? rows_in(a, b, g.nx - g.npml - 1, g.nx - 1) : 0;
+        const int e = (lo ? rows_in(a, b, 1, g.npml + 1) : 0) + upper, hh = (lo ? rows_in(a, b, 0, g.npml) : 0) + upper;
+        *smem = std::max(*smem, res2d_smem_bytes(job, a, b, e, hh, *shape));
+    }
+    if (*smem > (size_t)h->res_smem_limit) return OS_OK;
+    if (!h->res_row_start.ptr) OS_TRY(upload(h->res_row_start, h->res_rows.data(), h->res_rows.size(), h->stream));
+    if (!h->res_mail.ptr) {
+        OS_TRY(h->res_mail.alloc(res2d_mail_words(h->polarization, g.ny, (int)h->res_rows.size() - 1)));
+        OS_CUDA(cudaMemsetAsync(h->res_mail.ptr, 0, h->res_mail.bytes(), h->stream));
+        h->res_epoch = 1;
+    }
+    job.row_start = h->res_row_start.ptr;
+    job.mail = h->res_mail.ptr;
+    *yes = true;
+    return OS_OK;
+}
+
+// Resident launches of one device are ordered one after another, whatever their streams: each needs the whole chip,
+// and its blocks wait for one another.
+static int launch_resident(OsFdtd2D *h, const Res2DJob &job, int shape, size_t smem) {
+    static std::mutex mu;
+    static cudaEvent_t last[OS_FDTD_MAX_DEVICES] = {};
+    OS_CHECK(h->device >= 0 && h->device < OS_FDTD_MAX_DEVICES, OS_ERR_INVALID, "device %d is outside [0, %d)",
+             h->device, OS_FDTD_MAX_DEVICES);
+    std::lock_guard<std::mutex> lock(mu);
+    cudaEvent_t &ev = last[h->device];
+    if (ev) OS_CUDA(cudaStreamWaitEvent(h->stream, ev, 0));
+    else OS_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    OS_CUDA(res2d_launch(shape, job, smem, h->stream));
+    OS_CUDA(cudaEventRecord(ev, h->stream));
+    h->launches += 1;
+    return OS_OK;
+}
+
+// A chunk in the resident form: one launch per RES_STAGE_FLOATS of staged flux samples (normally one for the chunk),
+// then one fold per flux line.
+constexpr size_t RES_STAGE_FLOATS = (size_t)16 << 20;
+static int advance_resident(OsFdtd2D *h, Res2DJob job, int shape, size_t smem, int64_t n_steps, int64_t first_sample,
+                            int64_t n_samples, const float *values, const float *phase_table) {
+    const int64_t m = h->sample_interval;
+    size_t per_sample = 0;
+    for (auto &f : h->fluxes) per_sample += 2 * (size_t)(f->hi - f->lo);
+    const int64_t max_samples = per_sample ? std::max<int64_t>(1, (int64_t)(RES_STAGE_FLOATS / per_sample)) : 0;
+    job.values_stride = n_steps;
+    job.q_table = first_sample;
+    size_t offset = 0;
+    for (auto &f : h->fluxes) offset += (size_t)n_samples * f->nf * 2;
+    for (int k = 0; k < job.n_maps; ++k) {
+        ResMap &q = job.maps[k];
+        q.ph_e = phase_table + offset;
+        q.ph_h = q.ph_e + (size_t)n_samples * q.nf * 2;   // H_z engines: the second table of the map
+        offset += (size_t)n_samples * q.nf * 2 * (job.hz ? 2 : 1);
+    }
+    for (int64_t k = 0; k < n_steps;) {
+        int64_t n = n_steps - k;
+        if (max_samples) n = std::min(n, (h->n_step / m + max_samples + 1) * m - 1 - h->n_step);
+        const int64_t q_lo = h->n_step / m + 1, q_hi = (h->n_step + n) / m;
+        const bool sampled = !h->fluxes.empty() && q_hi >= q_lo;
+        if (sampled) OS_TRY(h->res_stage.alloc(per_sample * (size_t)(q_hi - q_lo + 1), h->stream));
+        job.n_mons = sampled ? (int32_t)h->fluxes.size() : 0;
+        float *stage = h->res_stage.ptr;
+        for (int f = 0; f < job.n_mons; ++f) {
+            const FluxLine2D &line = *h->fluxes[f];
+            job.mons[f] = ResMon{line.normal_axis, line.position, line.lo, line.hi, stage};
+            stage += 2 * (size_t)(line.hi - line.lo) * (size_t)(q_hi - q_lo + 1);
+        }
+        job.n_steps = n;
+        job.n0 = h->n_step;
+        job.q_first = q_lo;
+        job.epoch = h->res_epoch;
+        job.line_values = values + k;
+        for (int b = 0; b < job.n_tfsf; ++b) job.tfsf[b].values = values + (h->lines.size() + b) * (size_t)n_steps + k;
+        OS_TRY(launch_resident(h, job, shape, smem));
+        h->res_epoch += (uint32_t)n + 1u;
+        size_t at = 0;
+        for (int f = 0; f < job.n_mons; ++f) {
+            FluxLine2D &line = *h->fluxes[f];
+            const int cells_n = line.hi - line.lo, total = cells_n * line.nf;
+            ez2d_flux_staged_kernel<<<(total + 255) / 256, 256, 0, h->stream>>>(
+                job.mons[f].stage, cells_n, line.nf, (int)(q_hi - q_lo + 1), 0, 1,
+                phase_table + at + (size_t)(q_lo - first_sample) * line.nf * 2, line.e_acc.ptr, line.h_acc.ptr);
+            h->launches += 1;
+            at += (size_t)n_samples * line.nf * 2;
+        }
+        OS_CUDA(cudaGetLastError());
+        h->n_step += n;
+        k += n;
+    }
+    return OS_OK;
+}
+
 // Argument and state checks shared by the advance entry points (`fn` names the caller in messages).
 static int check_advance(const OsFdtd2D *h, const char *fn, int64_t n_steps, const float *line_values,
                          int64_t first_sample, int64_t n_samples, const float *phases) {
@@ -1819,10 +2038,17 @@ static int check_advance(const OsFdtd2D *h, const char *fn, int64_t n_steps, con
 
 // The chunk's kernels between the start/stop timing events, reading the given device tables.
 static int run_chunk(OsFdtd2D *h, int64_t n_steps, int64_t first_sample, int64_t n_samples, const float *values,
-                     const float *phase_table) {
+                     const float *phase_table, bool may_allocate = true) {
     OS_CUDA(cudaEventRecord(h->ev_start, h->stream));
+    bool resident = false;   // keeps strips, mail and staged samples of its own: not for a caller that must not allocate
+    Res2DJob job{};
+    int shape = -1;
+    size_t smem = 0;
+    if (may_allocate) OS_TRY(resident_applies(h, job, &shape, &smem, &resident));
     // a TFSF box or a pole acts between the H and E updates of every step: the per-half-step kernels run them
-    const int rc = h->polarization == 1 ? advance_hz(h, n_steps, first_sample, n_samples, values, phase_table)
+    const int rc = resident ? advance_resident(h, job, shape, smem, n_steps, first_sample, n_samples, values,
+                                               phase_table)
+                   : h->polarization == 1 ? advance_hz(h, n_steps, first_sample, n_samples, values, phase_table)
                    : (h->variant == 0 || !h->tfsf.empty() || !h->poles.empty())
                        ? advance_per_step(h, n_steps, first_sample, n_samples, values, phase_table)
                        : advance_blocked(h, n_steps, first_sample, n_samples, values, phase_table);
@@ -1946,7 +2172,7 @@ extern "C" int os_fdtd2d_advance_noalloc(OsFdtd2D *h, int64_t n_steps, const flo
     if (phase_floats)
         OS_CUDA(cudaMemcpyAsync(scratch + phase_offset, phases, phase_floats * sizeof(float),
                                 cudaMemcpyHostToDevice, h->stream));
-    return run_chunk(h, n_steps, first_sample, n_samples, scratch, scratch + phase_offset);
+    return run_chunk(h, n_steps, first_sample, n_samples, scratch, scratch + phase_offset, false);
 }
 
 extern "C" int os_fdtd2d_set_stall_probe(OsFdtd2D *h, int64_t wait_ns) {
@@ -1959,8 +2185,10 @@ extern "C" int os_fdtd2d_set_stall_probe(OsFdtd2D *h, int64_t wait_ns) {
 
 extern "C" int os_fdtd2d_configure(OsFdtd2D *h, int32_t variant, int32_t steps_per_launch, int32_t tile_rows) {
     OS_CHECK(h, OS_ERR_INVALID, "os_fdtd2d_configure: null handle");
-    OS_CHECK(variant >= 0 && variant <= 2, OS_ERR_INVALID,
-             "variant must be 0 (per half step), 1 (blocked) or 2 (blocked, general kernel only)");
+    OS_CHECK(variant >= 0 && variant <= 3, OS_ERR_INVALID,
+             "variant must be 0 (per half step), 1 (blocked), 2 (blocked, general kernel only) or 3 (automatic)");
+    const bool automatic = variant == 3;   // the resident form where it fits, else the blocked kernels
+    if (automatic) variant = 1;
     OS_CHECK(steps_per_launch >= 1 && steps_per_launch <= TB_MAX_T, OS_ERR_INVALID,
              "steps_per_launch must be in [1, %d], got %d", TB_MAX_T, steps_per_launch);
     if (h->polarization == 1) {
@@ -1984,12 +2212,14 @@ extern "C" int os_fdtd2d_configure(OsFdtd2D *h, int32_t variant, int32_t steps_p
             }
         }
         h->variant = variant;
+        h->automatic = automatic;
         h->steps_per_launch = steps_per_launch;
         h->hz_rows = tile_rows;
         return OS_OK;
     }
     OS_CHECK(tile_rows >= 0, OS_ERR_INVALID, "tile_rows must be >= 0 (0: chosen from the grid), got %d", tile_rows);
     h->variant = variant;
+    h->automatic = automatic;
     h->steps_per_launch = steps_per_launch;
     h->tile_rows = tile_rows;
     return OS_OK;

@@ -1,0 +1,6 @@
+// The resident kernels of the H_z engine, plain lossless runs (a file of their own to compile beside the others).
+#include "fdtd2d_resident_kernel.cuh"
+
+cudaError_t res2d_launch_hz_plain(int shape, const Res2DJob &job, size_t smem, cudaStream_t stream) {
+    return res_launch_any<true, false>(shape, job, smem, stream);
+}

@@ -56,7 +56,7 @@ class FDTDEngine2D_Ez:
         self._materials_version = None
         self.sample_interval = 1
         self._sample_interval_sent = None
-        self.variant, self.steps_per_launch, self.tile_rows = 1, 3, 0
+        self.variant, self.steps_per_launch, self.tile_rows = 3, 3, 0
         self._config_sent = None
         self.h2d_bytes = 0   # host-to-device bytes this engine has uploaded (setup, materials, chunk tables)
 
@@ -220,9 +220,13 @@ class FDTDEngine2D_Ez:
         """Kernel choice (results are bit-identical for every choice): variant 1 = temporally blocked kernels
         advancing steps_per_launch (1..4, default 3) steps per launch with tile_rows rows per interior tile (0, the
         default: chosen from the grid), the frame one step per launch; variant 2 = the same with the blocked general
-        kernel on the frame; variant 0 = one H and one E kernel per step."""
+        kernel on the frame; variant 0 = one H and one E kernel per step; variant 3 (a new engine's choice) = the whole
+        chunk in one launch with the fields in shared memory where the grid fits the chip, else variant 1.  Asking for
+        steps_per_launch or tile_rows alone picks the blocked kernels they belong to."""
         if variant is not None:
             self.variant = int(variant)
+        elif self.variant == 3 and (steps_per_launch is not None or tile_rows is not None):
+            self.variant = 1
         if steps_per_launch is not None:
             self.steps_per_launch = int(steps_per_launch)
         if tile_rows is not None:
@@ -433,7 +437,7 @@ class FDTDEngine2D_Hz(FDTDEngine2D_Ez):
 
     def __init__(self, domain, boundary_config, device: int = 0):
         super().__init__(domain, boundary_config, device)
-        self.variant, self.steps_per_launch, self.tile_rows = 1, 2, 0
+        self.variant, self.steps_per_launch, self.tile_rows = 3, 2, 0
         bc = boundary_config
         widths_x, widths_y = domain.kernel_widths()
         self.shares_x = face_shares(widths_x, bc.periodic_x)
@@ -471,8 +475,9 @@ class FDTDEngine2D_Hz(FDTDEngine2D_Ez):
         self.h2d_bytes += sum(a.nbytes for a in arrays if a is not None)
 
     def configure(self, variant=None, steps_per_launch=None, tile_rows=None):
-        """variant 1 (default): interior + border kernel per step, tile_rows interior rows per CTA (0 = chosen per
-        grid); variant 0: one H_z and one E kernel per step.  steps_per_launch 2 (default) or 1: with 2, where the grid
+        """variant 1: interior + border kernel per step, tile_rows interior rows per CTA (0 = chosen per grid); variant
+        0: one H_z and one E kernel per step; variant 3 (a new engine's choice): the whole chunk in one launch with the
+        fields in shared memory where the grid fits the chip, else variant 1.  steps_per_launch 2 (default) or 1: with 2, where the grid
         has no conductivity, no magnetic cells and rows of a multiple of 4 cells, the interior box advances two steps
         per launch (the border two single steps through a scratch field set, made here) except where the next step is
         a sampled one; a TFSF box or poles keep one step per launch."""

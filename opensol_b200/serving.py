@@ -144,7 +144,8 @@ def build_job(spec, device=0, steps_per_launch=3, tile_rows=0):
     freqs = np.linspace(0.8, 1.2, spec.n_freqs) * (2.99792458e8 / spec.wavelength)
     monitors = [sim.add_flux_monitor('y', frac * window, (0.0, window), frequencies=freqs.tolist())
                 for frac in (0.05, 0.9)]
-    sim.em.engine.configure(variant=1, steps_per_launch=steps_per_launch, tile_rows=tile_rows)
+    if tile_rows or steps_per_launch != 3:   # else the engine's own choice
+        sim.em.engine.configure(variant=1, steps_per_launch=steps_per_launch, tile_rows=tile_rows)
     sim.em.finalize()
     return sim, monitors
 

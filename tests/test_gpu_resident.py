@@ -1,0 +1,175 @@
+"""The resident form of the 2D step (a whole chunk in one launch, fields in shared memory; what a new engine runs where
+the grid fits) against the per-half-step kernels (variant 0), which the oracle and open_sol's fixtures pin: fields,
+spectra, maps and probe series bit for bit, on strips of one row and of many, every boundary preset, odd rows, lossy
+and magnetic cells, plane-wave boxes, poles, chunk ends on and off DFT samples, and switches between the forms."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import opensol_b200 as ob
+from opensol_b200 import _native
+
+pytestmark = pytest.mark.gpu
+DX = 20e-9
+
+
+def _sim(pol, nx, ny, boundaries, npml, seed, lossy=False, magnetic=False, tfsf=0, poles=(), maps=(), probes=0,
+         lines=('y', 'x')):
+    rng = np.random.default_rng(seed)
+    sim = ob.Simulation(nx * DX, ny * DX, DX, npml=npml, boundaries=boundaries, polarization=pol, verbose=False)
+    shape = (sim.grid.nx, sim.grid.ny)
+    materials = sim.domain.materials
+    for name in (('eps_r',) if pol == 'ez' else ('eps_xx', 'eps_yy')):
+        materials.array(name)[...] = rng.uniform(2.0, 6.0, shape)   # above the poles' stability term
+    if lossy:
+        materials.array('sigma_e')[...] = rng.uniform(0, 4e4, shape) * (rng.random(shape) < 0.3)
+    if magnetic:
+        materials.array('mu_r')[...] = rng.uniform(1.0, 2.0, shape)
+        materials.array('sigma_m')[...] = rng.uniform(0, 1e3, shape)
+    sim.em.materials_changed(('eps_r', 'eps_xx', 'eps_yy', 'sigma_e', 'mu_r', 'sigma_m'))
+    at = lambda cell: (cell + 0.5) * DX   # noqa: E731
+    for k, pole in enumerate(poles):
+        mask = np.zeros(shape, bool)
+        a, b = int(shape[0] * (0.3 + 0.1 * k)), int(shape[1] * 0.3)
+        mask[a:a + shape[0] // 4 + 1, b:b + shape[1] // 3 + 1] = rng.random((shape[0] // 4 + 1, shape[1] // 3 + 1)) < 0.8
+        sim.add_dispersive(pole, mask)
+    for k, axis in enumerate(lines):
+        n_across, n_along = (nx, ny) if axis == 'y' else (ny, nx)
+        span = None if k == 0 else (at(n_along // 5), at(4 * n_along // 5))
+        sim.add_line_source(axis, at(int(0.3 * n_across)), wavelength=700e-9, bandwidth=0.8, amplitude=1.0 + k,
+                            span=span)
+    for k in range(tfsf):
+        sim.add_tfsf(at(4 + k), at(5 + k), at(nx - 6), at(ny - 5 - k), wavelength=800e-9, bandwidth=0.5)
+    freqs = [3.5e14, 4.2e14, 5e14]
+    out = [sim.add_flux_monitor('y', at(int(f * nx)), (0.0, ny * DX), frequencies=freqs).spectra for f in (0.1, 0.8)]
+    out.append(sim.add_flux_monitor('x', at(int(0.7 * ny)), (at(1), at(nx - 2)), frequencies=freqs[:1]).spectra)
+    for ds in maps:
+        monitor = sim.add_dft_monitor(0.0, at(1), nx * DX, at(ny - 2), frequencies=freqs[:2], downsample=ds)
+        out.append(lambda m=monitor: m._maps())
+    components = ('ez', 'hx', 'hy') if pol == 'ez' else ('hz', 'ex', 'ey')
+    for k in range(probes):
+        probe = sim.add_field_probe(at(int((0.2 + 0.29 * k) * nx)), at(int((0.8 - 0.3 * k) * ny)), components[k % 3])
+        out.append(lambda p=probe: p.get_data()[1])
+    sim.finalize()
+    start = np.random.default_rng(seed + 1)
+    for name in sim.em.engine.FIELDS:
+        scale = 1.0 if name[0] == 'e' else 2.7e-3
+        sim.em.engine.write_field(name, (scale * start.standard_normal(shape)).astype(np.float32))
+    return sim, out
+
+
+def _outputs(sim, out):
+    engine = sim.em.engine
+    got = [engine.read_field(name) for name in engine.FIELDS]
+    for read in out:
+        value = read()
+        got.extend(value if isinstance(value, tuple) else [value])
+    return got
+
+
+def _compare(args, chunks, switch=None):
+    """chunks of steps in the resident form and in variant 0 from the same seeded fields; `switch`: after that chunk the
+    resident engine continues with the blocked kernels and then goes back."""
+    sim, out = _sim(**args)
+    ref, ref_out = _sim(**args)
+    ref.em.engine.configure(variant=0)
+    for k, n in enumerate(chunks):
+        if switch is not None and k in (switch, switch + 1):
+            sim.em.engine.configure(variant=1 if k == switch else 3)
+        sim.em.engine.advance(n)
+        launches = sim.em.engine.launch_count()
+        if switch is None or k != switch:
+            assert launches <= 1 + 3   # one resident launch, one fold per flux line
+        ref.em.engine.advance(n)
+    for a, b in zip(_outputs(sim, out), _outputs(ref, ref_out)):
+        np.testing.assert_array_equal(a, b)
+        assert np.isfinite(np.asarray(b)).all()
+    assert np.abs(_outputs(sim, out)[0]).max() > 0
+
+
+DRUDE, LORENTZ = ob.DrudePole(6e15, 2e14), ob.LorentzPole(1.5, 5e15, 3e14)
+CASES = [
+    dict(nx=120, ny=75, boundaries='pml', npml=10),
+    dict(nx=127, ny=64, boundaries='pml', npml=10, lossy=True, probes=3),            # 147 strips of one row
+    dict(nx=129, ny=33, boundaries='pml', npml=10, magnetic=True, probes=2),         # 149 rows: strips of one and two
+    dict(nx=300, ny=1200, boundaries='pml', npml=15, maps=(3,)),                     # several columns a thread
+    dict(nx=777, ny=129, boundaries='periodic_y', npml=15, maps=(1,), probes=1),
+    dict(nx=150, ny=131, boundaries='periodic_x', npml=8, lines=('x', 'y'), maps=(2,)),
+    dict(nx=149, ny=90, boundaries='periodic', npml=15, lossy=True, magnetic=True),
+    dict(nx=160, ny=140, boundaries='pml', npml=12, tfsf=1, lines=(), poles=(DRUDE, LORENTZ), probes=1),
+    dict(nx=90, ny=141, boundaries='periodic_y', npml=9, poles=(DRUDE, DRUDE, LORENTZ), lossy=True, maps=(2,)),
+    dict(nx=330, ny=77, boundaries='periodic_x', npml=9, lines=('x',), poles=(LORENTZ,), tfsf=2),
+]
+
+
+@pytest.mark.parametrize('pol', ['ez', 'hz'])
+@pytest.mark.parametrize('case', range(len(CASES)))
+def test_resident_equals_per_step(pol, case):
+    args = dict(CASES[case], pol=pol, seed=100 + case)
+    _compare(args, (41, 1, 2, 36))
+
+
+@pytest.mark.parametrize('pol', ['ez', 'hz'])
+def test_resident_among_the_other_forms(pol):
+    """Chunks in the resident form, then blocked, then resident again continue one run."""
+    _compare(dict(pol=pol, nx=200, ny=164, boundaries='pml', npml=10, seed=7, maps=(3,), probes=2), (20, 31, 25), 1)
+
+
+def test_resident_two_rows():
+    """The smallest strips: a periodic grid of 2 x 40 cells, and of 3 rows."""
+    for nx in (2, 3):
+        sim, out = {}, {}
+        for variant in (3, 0):
+            s = ob.Simulation(nx * DX, 40 * DX, DX, boundaries='periodic', verbose=False)
+            s.add_line_source('x', 10.5 * DX, wavelength=700e-9)
+            s.em.engine.configure(variant=variant)
+            s.run(n_steps=55, verbose=False)
+            sim[variant], out[variant] = s, [s.em.engine.read_field(n) for n in ('ez', 'hx', 'hy')]
+        for a, b in zip(out[3], out[0]):
+            np.testing.assert_array_equal(a, b)
+        assert np.abs(out[0][0]).max() > 0
+
+
+def test_resident_engines_share_the_device():
+    """Engines on streams of their own advanced from the host in turn: each launch needs the whole chip, and every
+    result is that of the engine alone."""
+    args = [dict(pol=p, nx=180, ny=100, boundaries='pml', npml=10, seed=s) for p, s in (('ez', 1), ('hz', 2), ('ez', 3))]
+    together = [_sim(**a) for a in args]
+    for _ in range(3):
+        for sim, _out in together:
+            sim.em.engine.advance(40)
+    for a, (sim, out) in zip(args, together):
+        alone, alone_out = _sim(**a)
+        for _ in range(3):
+            alone.em.engine.advance(40)
+        for x, y in zip(_outputs(sim, out), _outputs(alone, alone_out)):
+            np.testing.assert_array_equal(x, y)
+
+
+def test_resident_bounded_wait():
+    """A boundary row that never arrives (the test hook: one strip sends none for 1 ms and leaves) ends the launch with
+    the error status; the engine runs again after a reset."""
+    args = dict(pol='ez', nx=150, ny=100, boundaries='pml', npml=10, seed=4)
+    sim, out = _sim(**args)
+    engine = sim.em.engine
+    engine.set_stall_probe(1_000_000)
+    engine.advance(30)
+    with pytest.raises(RuntimeError, match='bounded wait'):
+        engine.synchronize()
+    engine.set_stall_probe(0)
+    engine.reset()
+    engine.advance(30)
+    engine.synchronize()
+    clean, clean_out = _sim(**args)
+    clean.em.engine.reset()
+    clean.em.engine.advance(30)
+    for a, b in zip(_outputs(sim, out), _outputs(clean, clean_out)):
+        np.testing.assert_array_equal(a, b)
+
+
+def test_variant_range_is_refused():
+    sim, _ = _sim(pol='ez', nx=40, ny=40, boundaries='pml', npml=8, seed=1)
+    for variant in (-1, 4):
+        with pytest.raises(ValueError):
+            _native.check(_native.load().os_fdtd2d_configure(sim.em.engine.handle, ctypes.c_int32(variant), 3, 0))
