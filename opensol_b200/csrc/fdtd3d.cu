@@ -22,6 +22,7 @@
 #include "fdtd3d_lean.cuh"
 
 #include <algorithm>
+#include <cmath>
 #include <memory>
 #include <vector>
 
@@ -67,7 +68,8 @@ struct OsFdtd3D {
     int64_t sample_interval = 1;
     int64_t n_step = 0;
     int64_t launches = 0;
-    int32_t x_chunk = 64;
+    int32_t x_chunk = 64;          // planes a block of the fused forms streams
+    int32_t in_place_chunk = 64;   // and of the two in-place kernels
     os::DeviceArray<float> values;              // (n_dipoles, n_steps) of the current chunk
     os::DeviceArray<float> phases;              // (n_samples, sum nf, 2) of the current chunk
     os::DeviceArray<float> scratch;             // one float (face cb read-back)
@@ -516,9 +518,14 @@ extern "C" int os_fdtd3d_create(const OsGrid3D *grid, OsFdtd3D **out) {
     OS_TRY(h->scratch.alloc(1));
     OS_TRY(h->err.alloc(1));
     OS_CUDA(cudaMemsetAsync(h->err.ptr, 0, sizeof(int32_t), h->stream));
-    // x chunk: short runs of 24 planes per block (many more blocks than resident slots, so the last wave is a small
-    // share of the launch; on 512^3 the step ran 37.9 G cell-updates/s at 256 planes, 48.6-50.4 at 12-32)
+    // Planes a block streams.  Long runs read fewer planes twice, short ones give enough blocks to fill the chip (at
+    // 512^3 24 planes ran 48.6-50.4 G cell-updates/s, 256 planes 37.9).  The in-place kernels, which small grids run, are
+    // best at sqrt(column blocks x planes / 1000) planes, at most 24: us per step at 24 planes and at this length,
+    // 75 x 75 x 165 cells 63.8 and 33.2, 144 x 134 x 124 113 and 80.6, 250 x 230 x 145 239 and 218.
     h->x_chunk = std::min<int32_t>(g.nx, 24);
+    const double column_blocks = std::ceil((double)g.nz / EM3D_BZ) * std::ceil((double)g.ny / EM3D_BY);
+    const int32_t planes = (int32_t)std::lround(std::sqrt(column_blocks * g.nx / 1000.0));
+    h->in_place_chunk = std::min<int32_t>(g.nx, std::max<int32_t>(1, std::min<int32_t>(24, planes)));
     OS_TRY(zero_state3(h.get()));
     OS_CUDA(cudaStreamSynchronize(h->stream));
     *out = h.release();
@@ -776,6 +783,10 @@ extern "C" int os_fdtd3d_advance(OsFdtd3D *h, int64_t n_steps, const float *dipo
             if (c.nr && !c.psi2.ptr) OS_TRY(c.psi2.alloc(4 * c.psi_count));
     }
     Em3DParams p = make_params3(h);
+    if (!fused) {
+        p.x_chunk = h->in_place_chunk;
+        whole_grid_boxes(h, p);
+    }
     p.dip_values = h->values.ptr;
     p.values_stride = n_steps;
     Em3DParams pd = p;   // the lean form adds the dipoles after the step, in em3d_dipole_kernel
@@ -897,7 +908,7 @@ extern "C" int os_fdtd3d_set_stream(OsFdtd3D *h, void *cuda_stream) {
 extern "C" int os_fdtd3d_set_x_chunk(OsFdtd3D *h, int32_t planes) {
     OS_CHECK(h, OS_ERR_INVALID, "os_fdtd3d_set_x_chunk: null handle");
     OS_CHECK(planes >= 1, OS_ERR_INVALID, "x chunk must be >= 1 plane, got %d", planes);
-    h->x_chunk = planes;
+    h->x_chunk = h->in_place_chunk = planes;
     return OS_OK;
 }
 
