@@ -518,11 +518,14 @@ extern "C" int os_fdtd3d_create(const OsGrid3D *grid, OsFdtd3D **out) {
     OS_TRY(h->scratch.alloc(1));
     OS_TRY(h->err.alloc(1));
     OS_CUDA(cudaMemsetAsync(h->err.ptr, 0, sizeof(int32_t), h->stream));
-    // Planes a block streams.  Long runs read fewer planes twice, short ones give enough blocks to fill the chip (at
-    // 512^3 24 planes ran 48.6-50.4 G cell-updates/s, 256 planes 37.9).  The in-place kernels, which small grids run, are
-    // best at sqrt(column blocks x planes / 1000) planes, at most 24: us per step at 24 planes and at this length,
-    // 75 x 75 x 165 cells 63.8 and 33.2, 144 x 134 x 124 113 and 80.6, 250 x 230 x 145 239 and 218.
-    h->x_chunk = std::min<int32_t>(g.nx, 24);
+    // Planes a block streams.  Long runs read fewer planes twice, short ones give enough blocks to fill the chip.  The
+    // fused forms: 1/22 of the grid's mean extent, 4 to 24, evened out over the chunks (lean form, us per step at 24
+    // planes and at 8: 160^3 207 and 178, 240 x 224 x 256 350 and 303; 384^3 896 at 24 and 879 at 16; 512^3 keeps 23).
+    // The in-place kernels, which other small grids run: sqrt(column blocks x planes / 1000), at most 24 (at 24 planes
+    // and at this length: 75 x 75 x 165 cells 63.8 and 33.2, 144 x 134 x 124 113 and 80.6, 250 x 230 x 145 236 and 215).
+    const int32_t extent = std::max(4, std::min(24, (int)std::lround(std::cbrt((double)n) / 22.0)));
+    const int32_t chunks = (g.nx + extent - 1) / extent;
+    h->x_chunk = std::min<int32_t>(g.nx, (g.nx + chunks - 1) / chunks);
     const double column_blocks = std::ceil((double)g.nz / EM3D_BZ) * std::ceil((double)g.ny / EM3D_BY);
     const int32_t planes = (int32_t)std::lround(std::sqrt(column_blocks * g.nx / 1000.0));
     h->in_place_chunk = std::min<int32_t>(g.nx, std::max<int32_t>(1, std::min<int32_t>(24, planes)));
