@@ -53,10 +53,13 @@ __host__ __device__ static inline int res_coef_arrays(const Res2DJob &p) {
 }
 __host__ __device__ static inline size_t res_mail_rows(int hz) { return hz ? 3 : 2; }
 
-// Words of shared memory (floats) one strip's poles take: per pole drive and state of its rows in the strip.
-__host__ __device__ static inline int res_pole_floats(const ResPole &q, int i0, int i1) {
+// A pole's rows in shared memory: the columns of the threads (c each) its box reaches, drive and state (2 or 3 arrays).
+__host__ __device__ static inline int res_pole_width(const ResPole &q, int c) {
+    return ((q.j1 + c - 1) / c - q.j0 / c) * c;
+}
+__host__ __device__ static inline int res_pole_floats(const ResPole &q, int i0, int i1, int c) {
     const int a = q.i0 > i0 ? q.i0 : i0, b = q.i1 < i1 ? q.i1 : i1;
-    return b > a ? (b - a) * (q.j1 - q.j0) * (q.kind == 0 ? 2 : 3) : 0;
+    return b > a ? (b - a) * res_pole_width(q, c) * (q.kind == 0 ? 2 : 3) : 0;
 }
 
 __device__ __forceinline__ float2 rs_sub(float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
@@ -167,131 +170,150 @@ static __device__ __noinline__ void res_maps_hz(const Res2DJob &p, int i, int j,
     }
 }
 
-// Plane-wave box corrections of a thread's columns j0 .. j0 + C - 1 on row i; aux: the boxes' incident E cells, then H
-// cells, box after box.  `v` and `w`: H_x and H_y after the H update, or E_z (w unused) after the E update, of an E_z
-// engine; H_z (w unused) after its update, or E_x and E_y after theirs, of an H_z engine.
-struct ResPair4 {
-    float4 v, w;
-};
+extern __shared__ __align__(16) unsigned char res_smem[];   // the block's shared memory (functions that are not inlined
+                                                            // address it by offset, so their accesses stay shared ones)
+
+// Plane-wave boxes: each box's incident line in shared memory is four arrays of aux_n floats at `at`: E cells, H cells
+// and their coefficients.  The corrections of the boxes' x sides on a thread's columns j0 .. j0 + C - 1 of row i (the y
+// sides are ResStrip::tfsf_columns'): `v` is H_y after the H update or E_z after the E update of an E_z engine, H_z after
+// its update or E_y after the E update of an H_z engine.
 template <int C>
-static __device__ __noinline__ ResPair4 res_tfsf(const Res2DJob &p, const float *aux, bool e_phase, int i, int j0,
-                                                 ResPair4 in) {
-    float v[4] = {in.v.x, in.v.y, in.v.z, in.v.w}, w[4] = {in.w.x, in.w.y, in.w.z, in.w.w};
+static __device__ __noinline__ float4 res_tfsf_row(const Res2DJob &p, int at, bool e_phase, int i, int j0, float4 in) {
+    float v[4] = {in.x, in.y, in.z, in.w};
 #pragma unroll 1
     for (int k = 0; k < p.n_tfsf; ++k) {
         const ResTfsf &t = p.tfsf[k];
-        const float *h = aux + t.aux_n;
-        const int last = t.aux_x0 + (t.x1 - 1 - t.x0), along = t.aux_x0 + (i - t.x0);
-        const bool in_x = i >= t.x0 && i < t.x1;
+        const float *e = reinterpret_cast<const float *>(res_smem) + at, *h = e + t.aux_n;
+        const int last = t.aux_x0 + (t.x1 - 1 - t.x0);
+        float lo = 0.0f, hi = 0.0f;   // signed terms of the two sides
+        bool on_lo, on_hi;
+        if (!p.hz && !e_phase) {
+            on_lo = i == t.x0 - 1, lo = -(t.coef_h[0] * e[t.aux_x0]);
+            on_hi = i == t.x1 - 1, hi = t.coef_h[1] * e[last];
+        } else if (!p.hz) {
+            on_lo = i == t.x0, lo = -(t.coef_e[0] * h[t.aux_x0 - 1]);
+            on_hi = i == t.x1 - 1, hi = t.coef_e[1] * h[last];
+        } else if (!e_phase) {
+            on_lo = i == t.x0, lo = t.coef_h[0] * e[t.aux_x0 - 1];
+            on_hi = i == t.x1 - 1, hi = -(t.coef_h[1] * e[last]);
+        } else {
+            on_lo = i == t.x0 - 1, lo = t.coef_e[0] * h[t.aux_x0];
+            on_hi = i == t.x1 - 1, hi = -(t.coef_e[1] * h[last]);
+        }
 #pragma unroll
         for (int c = 0; c < C; ++c) {
-            const int j = j0 + c;
-            const bool in_y = j >= t.y0 && j < t.y1;
-            if (!p.hz && !e_phase) {
-                if (in_y && i == t.x0 - 1) w[c] = w[c] - t.coef_h[0] * aux[t.aux_x0];
-                if (in_y && i == t.x1 - 1) w[c] = w[c] + t.coef_h[1] * aux[last];
-                if (in_x && j == t.y0 - 1) v[c] = v[c] + t.coef_h[2] * aux[along];
-                if (in_x && j == t.y1 - 1) v[c] = v[c] - t.coef_h[3] * aux[along];
-            } else if (!p.hz) {
-                if (in_y && i == t.x0) v[c] = v[c] - t.coef_e[0] * h[t.aux_x0 - 1];
-                if (in_y && i == t.x1 - 1) v[c] = v[c] + t.coef_e[1] * h[last];
-            } else if (!e_phase) {
-                if (in_y && i == t.x0) v[c] = v[c] + t.coef_h[0] * aux[t.aux_x0 - 1];
-                if (in_y && i == t.x1 - 1) v[c] = v[c] - t.coef_h[1] * aux[last];
-            } else {
-                if (in_y && i == t.x0 - 1) w[c] = w[c] + t.coef_e[0] * h[t.aux_x0];
-                if (in_y && i == t.x1 - 1) w[c] = w[c] - t.coef_e[1] * h[last];
-                if (in_x && j == t.y0 - 1) v[c] = v[c] - t.coef_e[2] * h[along];
-                if (in_x && j == t.y1 - 1) v[c] = v[c] + t.coef_e[3] * h[along];
-            }
+            if (j0 + c < t.y0 || j0 + c >= t.y1) continue;
+            if (on_lo) v[c] = v[c] + lo;
+            if (on_hi) v[c] = v[c] + hi;
         }
-        aux += 2 * t.aux_n;
+        at += 4 * t.aux_n;
     }
-    return ResPair4{make_float4(v[0], v[1], v[2], v[3]), make_float4(w[0], w[1], w[2], w[3])};
+    return make_float4(v[0], v[1], v[2], v[3]);
 }
 // The incident lines' half steps, by every block for itself (first phase: H from E, second: E from H, the soft source
 // and the Mur ends).  An H_z engine's H cells are shifted by one: H_z[k] from E_y[k] - E_y[k - 1], k >= 1.
-static __device__ __noinline__ void res_aux_h(const Res2DJob &p, float *aux, int tid, int nt) {
+static __device__ __noinline__ void res_aux_h(const Res2DJob &p, int at, int tid, int nt) {
     for (int k = 0; k < p.n_tfsf; ++k) {
-        const ResTfsf &t = p.tfsf[k];
-        float *h = aux + t.aux_n + (p.hz ? 1 : 0);
-        for (int a = tid; a < t.aux_n - 1; a += nt) h[a] = h[a] + __ldg(t.aux_coef_h + a) * (aux[a + 1] - aux[a]);
-        aux += 2 * t.aux_n;
+        const int n = p.tfsf[k].aux_n;
+        float *e = reinterpret_cast<float *>(res_smem) + at, *h = e + n + (p.hz ? 1 : 0);
+        const float *coef = e + 2 * n;
+        for (int a = tid; a < n - 1; a += nt) h[a] = h[a] + coef[a] * (e[a + 1] - e[a]);
+        at += 4 * n;
     }
 }
-static __device__ __noinline__ void res_aux_e(const Res2DJob &p, float *aux, int64_t k_step, int tid, int nt) {
+static __device__ __noinline__ void res_aux_e(const Res2DJob &p, int at, int64_t k_step, int tid, int nt) {
     for (int k = 0; k < p.n_tfsf; ++k) {
         const ResTfsf &t = p.tfsf[k];
-        const float *h = aux + t.aux_n + (p.hz ? 1 : 0);
         const int n = t.aux_n;
+        float *e = reinterpret_cast<float *>(res_smem) + at;
+        const float *h = e + n + (p.hz ? 1 : 0), *coef = e + 3 * n;
         for (int a = 1 + tid; a < n - 1; a += nt) {
-            const float old = aux[a];
-            float v = old + __ldg(t.aux_coef_e + a) * (h[a] - h[a - 1]);
+            const float old = e[a];
+            float v = old + coef[a] * (h[a] - h[a - 1]);
             if (a == t.source_index) v = v + __ldg(t.values + k_step);
-            aux[a] = v;
-            if (a == 1) aux[0] = old + t.mur_lo * (v - aux[0]);
-            if (a == n - 2) aux[n - 1] = old + t.mur_hi * (v - aux[n - 1]);
+            e[a] = v;
+            if (a == 1) e[0] = old + t.mur_lo * (v - e[0]);
+            if (a == n - 2) e[n - 1] = old + t.mur_hi * (v - e[n - 1]);
         }
-        aux += 2 * n;
+        at += 4 * n;
     }
 }
 
-// A pole's rows in the strip: its drive and state arrays in shared memory (drive, a, and b of a Lorentz pole, n floats
-// apart), first strip row, columns [j0, j1).
+// A pole's rows in the strip (floats from res_smem): drive, a, and b of a Lorentz pole, n floats apart, rows of w floats
+// from column c0; strip rows from `first`; the box's columns [j0, j1).
 struct __align__(16) ResPoleRows {
-    float *drive;
-    int32_t n, first, j0, j1, kind, comp;
+    int32_t at, n, first, w;
+    int32_t c0, j0, j1, kind;
     float damping, restoring;
+    int32_t comp, pad;
 };
-// Poles `mask` of the strip's table on a thread's columns of strip row r: the update from the field before the step
-// (fdtd_ez_2d.py:318-345).  The table lists Drude poles first, each kind in add order.
+// Poles `mask` of the strip's table on a thread's columns of strip row r: the update from the fields before the step
+// (fdtd_ez_2d.py:318-345): e0 is E_z, or E_x and e1 E_y.  The table lists Drude poles first, each kind in add order.
 template <int C>
-static __device__ __noinline__ void res_pole_update(const ResPoleRows *tab, uint32_t mask, int comp, int r, int j0,
-                                                    float4 e4) {
-    const float e[4] = {e4.x, e4.y, e4.z, e4.w};
+static __device__ __noinline__ void res_pole_update(int tab, uint32_t mask, int r, int j0, float4 e0, float4 e1) {
 #pragma unroll 1
     for (; mask; mask &= mask - 1) {
-        const ResPoleRows q = tab[__ffs(mask) - 1];
-        if (comp >= 0 && q.comp != comp) continue;
-        float *drive = q.drive + (r - q.first) * (q.j1 - q.j0) + (j0 - q.j0), *a = drive + q.n, *b = a + q.n;
+        const ResPoleRows q = reinterpret_cast<const ResPoleRows *>(res_smem + tab)[__ffs(mask) - 1];
+        const float4 e4 = q.comp ? e1 : e0;
+        const float e[4] = {e4.x, e4.y, e4.z, e4.w};
+        float2 *drive = reinterpret_cast<float2 *>(reinterpret_cast<float *>(res_smem) + q.at + (r - q.first) * q.w +
+                                                   (j0 - q.c0));
+        float2 *a = drive + q.n / 2, *b = a + q.n / 2;
+        float2 d2[C / 2], a2[C / 2], b2[C / 2];
+#pragma unroll
+        for (int k = 0; k < C / 2; ++k) {
+            d2[k] = drive[k], a2[k] = a[k];
+            if (q.kind) b2[k] = b[k];
+        }
 #pragma unroll
         for (int c = 0; c < C; ++c) {
             if (j0 + c < q.j0 || j0 + c >= q.j1) continue;
+            const float dr = (c & 1) ? d2[c >> 1].y : d2[c >> 1].x;
+            float &av = (c & 1) ? a2[c >> 1].y : a2[c >> 1].x;
             if (q.kind == 0) {
-                a[c] = a[c] + (q.damping * a[c] + drive[c] * e[c]);
+                av = av + (q.damping * av + dr * e[c]);
             } else {
-                const float dp = b[c] + (q.damping * b[c] - q.restoring * a[c] + drive[c] * e[c]);
-                b[c] = dp;
-                a[c] = a[c] + dp;
+                float &bv = (c & 1) ? b2[c >> 1].y : b2[c >> 1].x;
+                bv = bv + (q.damping * bv - q.restoring * av + dr * e[c]);
+                av = av + bv;
             }
+        }
+#pragma unroll
+        for (int k = 0; k < C / 2; ++k) {
+            a[k] = a2[k];
+            if (q.kind) b[k] = b2[k];
         }
     }
 }
-// Correction of the updated field.  E_z (comp < 0): the Drude total (the J itself when there is one Drude pole, else
-// summed from 0 in add order), then each Lorentz pole (fdtd_ez_2d.py:347-358; cells in no Drude box keep v, which is
-// v - cb * 0).  H_z: Drude sets, then Lorentz sets (fdtd_hz_2d.py:311-325).
+// Correction of the updated field of component comp (E_z: 0).  E_z: the Drude total (the J itself when there is one
+// Drude pole, else summed from 0 in add order), then each Lorentz pole (fdtd_ez_2d.py:347-358; cells in no Drude box keep
+// v, which is v - cb * 0).  H_z: Drude sets, then Lorentz sets (fdtd_hz_2d.py:311-325).
 template <int C>
-static __device__ __noinline__ float4 res_pole_correct(const ResPoleRows *tab, uint32_t mask, int comp, bool one_drude,
+static __device__ __noinline__ float4 res_pole_correct(int tab, uint32_t mask, bool hz, int comp, bool one_drude,
                                                        float inv_dt, int r, int j0, float4 v4, float4 cb4) {
     float v[4] = {v4.x, v4.y, v4.z, v4.w}, total[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     const float cb[4] = {cb4.x, cb4.y, cb4.z, cb4.w};
-    bool sum = comp < 0;   // the Drude total is still being summed
+    bool sum = !hz;   // the Drude total is still being summed
 #pragma unroll 1
     for (;; mask &= mask - 1) {
-        const ResPoleRows q = tab[mask ? __ffs(mask) - 1 : 0];
+        const ResPoleRows q = reinterpret_cast<const ResPoleRows *>(res_smem + tab)[mask ? __ffs(mask) - 1 : 0];
         if (sum && (!mask || q.kind == 1)) {
 #pragma unroll
             for (int c = 0; c < C; ++c) v[c] = v[c] - cb[c] * total[c];
             sum = false;
         }
         if (!mask) break;
-        if (comp >= 0 && q.comp != comp) continue;
-        const float *s = q.drive + (q.kind == 0 ? q.n : 2 * q.n) + (r - q.first) * (q.j1 - q.j0) + (j0 - q.j0);
+        if (q.comp != comp) continue;
+        const float2 *s2 = reinterpret_cast<const float2 *>(reinterpret_cast<const float *>(res_smem) + q.at +
+                                                            (q.kind == 0 ? q.n : 2 * q.n) + (r - q.first) * q.w +
+                                                            (j0 - q.c0));
+        const float scale = q.kind == 0 ? 1.0f : inv_dt;
 #pragma unroll
         for (int c = 0; c < C; ++c) {
+            const float s = (c & 1) ? s2[c >> 1].y : s2[c >> 1].x;
             if (j0 + c < q.j0 || j0 + c >= q.j1) continue;
-            if (sum) total[c] = one_drude ? s[c] : total[c] + s[c];
-            else v[c] = v[c] - cb[c] * (q.kind == 0 ? 1.0f : inv_dt) * s[c];
+            if (sum) total[c] = one_drude ? s : total[c] + s;
+            else v[c] = v[c] - cb[c] * scale * s;
         }
     }
     return make_float4(v[0], v[1], v[2], v[3]);
@@ -336,8 +358,8 @@ struct ResStrip {
     float *yeq, *yhq, *gy;         // y-side psi (R, Y: the layer threads' columns); the recomputed row's
     float *yrec;                   // y-side recursion: b, a, inv of the E kind, then of the H kind (Y each)
     int Y;
-    float *aux, *pole;
-    ResPoleRows *pole_rows;
+    int aux, pole_tab;             // incident lines (floats from res_smem), the pole table (bytes)
+    float *pole;
     int *dead;
     // fields
     float2 f[RT][H], a[RT][H], b[RT][H];
@@ -575,51 +597,75 @@ struct ResStrip {
             ez_hy(-1, row, got[0], ed, dbv, dav, gx, g);
         }
         if (GEN && p.n_tfsf) {
-            tfsf_ab(false);
-            if (has_up && (rows[0].flags & RF_EDGE)) {
-                const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                res_to(g, res_tfsf<C>(p, aux, false, rows[0].i, j0, ResPair4{zero, res_from(g)}).w);
-            }
+            tfsf_ab();
+            if (has_up && (rows[0].flags & RF_EDGE)) res_to(g, res_tfsf_row<C>(p, aux, false, rows[0].i, j0, res_from(g)));
         }
         publish_hi(a);
     }
 
-    // plane-wave box corrections of both in-plane fields on the boxes' edge rows and columns
-    __device__ __forceinline__ void tfsf_ab(bool e_phase) {
+    // plane-wave box corrections of the in-plane fields: b on the boxes' edge rows, a on their edge columns (from the
+    // incident E after the H update of an E_z engine, from the incident H after the E update of an H_z engine)
+    __device__ __forceinline__ void tfsf_ab() {
 #pragma unroll 1
         for (int r = 0; r < R; ++r) {
-            if (!edge_col && !(rows[r + 1].flags & RF_EDGE)) continue;
-            float2 x[H], y[H];
-            get(x, a, r);
+            if (!(rows[r + 1].flags & RF_EDGE)) continue;
+            float2 y[H];
             get(y, b, r);
-            const ResPair4 out = res_tfsf<C>(p, aux, e_phase, i0 + r, j0, ResPair4{res_from(x), res_from(y)});
-            res_to(x, out.v);
-            res_to(y, out.w);
-            put(a, x, r);
+            res_to(y, res_tfsf_row<C>(p, aux, HZ, i0 + r, j0, res_from(y)));
             put(b, y, r);
+        }
+        if (!edge_col) return;
+        const float *line = reinterpret_cast<const float *>(res_smem) + aux;
+#pragma unroll 1
+        for (int k = 0; k < p.n_tfsf; ++k) {
+            const ResTfsf &t = p.tfsf[k];
+            const float *incident = line + (HZ ? t.aux_n : 0) + t.aux_x0 + (i0 - t.x0);
+#pragma unroll
+            for (int side = 0; side < 2; ++side) {
+                const int at = (side ? t.y1 : t.y0) - 1 - j0;
+                if (at < 0 || at >= C) continue;
+                const float coef = HZ ? t.coef_e[2 + side] : t.coef_h[2 + side];
+                const bool minus = HZ ? side == 0 : side == 1;
+#pragma unroll
+                for (int r = 0; r < RT; ++r) {
+                    if (r >= R || i0 + r < t.x0 || i0 + r >= t.x1) continue;
+                    const float term = coef * incident[r], x = rs_get(a[r], at);
+                    rs_set(a[r], at, minus ? x - term : x + term);
+                }
+            }
+            line += 4 * t.aux_n;
         }
     }
 
-    // poles on the pole rows of a field: the updates from E^n before the E update, the corrections after it
-    __device__ __forceinline__ void poles(float2 (&v)[RT][H], int comp, const float *cb_rows, bool correct) {
+    // poles on the strip's pole rows: the updates from E^n before the E update (u: E_z or E_x, w: E_y of an H_z engine) ...
+    __device__ __forceinline__ void pole_updates(const float2 (&u)[RT][H], const float2 (&w)[RT][H]) {
+#pragma unroll 1
+        for (int r = 0; r < R; ++r) {
+            const uint32_t mask = rows[r + 1].poles & pole_mask;
+            if (!mask) continue;
+            float2 x[H], y[H];
+            get(x, u, r);
+            get(y, w, r);
+            res_pole_update<C>(pole_tab, mask, r, j0, res_from(x), res_from(y));
+        }
+    }
+    // ... and the corrections after it
+    __device__ __forceinline__ void pole_corrections(float2 (&v)[RT][H], int comp, const float *cb_rows) {
 #pragma unroll 1
         for (int r = 0; r < R; ++r) {
             const uint32_t mask = rows[r + 1].poles & pole_mask;
             if (!mask) continue;
             float2 x[H], cb[H];
             get(x, v, r);
-            if (!correct) {
-                res_pole_update<C>(pole_rows, mask, comp, r, j0, res_from(x));
-                continue;
-            }
             coef(cb, cb_rows, r);
-            res_to(x, res_pole_correct<C>(pole_rows, mask, comp, p.n_drude == 1, p.inv_dt, r, j0, res_from(x), res_from(cb)));
+            res_to(x, res_pole_correct<C>(pole_tab, mask, HZ, comp, p.n_drude == 1, p.inv_dt, r, j0, res_from(x),
+                                          res_from(cb)));
             put(v, x, r);
         }
     }
 
     __device__ __forceinline__ void ez_e(int64_t step, uint32_t epoch) {
-        if (GEN && pole_mask) poles(f, -1, cx, false);
+        if (GEN && pole_mask) pole_updates(f, f);
 #pragma unroll
         for (int r = 0; r < RT; ++r) {
             if (r >= R) break;
@@ -640,7 +686,7 @@ struct ResStrip {
             if (row.xe >= 0) x_layer(xe + row.xe * P, row.b_e, row.a_e, row.i_e, dx, cb, false, f[r]);
             if (ye) y_layer(yeq + r * Y, true, dy, cb, true, f[r]);
         }
-        if (GEN && pole_mask) poles(f, -1, cx, true);
+        if (GEN && pole_mask) pole_corrections(f, 0, cx);
         if (lines) sources(-1, step - 1, f);
         if (GEN && p.n_tfsf) {
 #pragma unroll 1
@@ -648,8 +694,7 @@ struct ResStrip {
                 if (!(rows[r + 1].flags & RF_TFSF)) continue;
                 float2 x[H];
                 get(x, f, r);
-                const float4 v = res_from(x);
-                res_to(x, res_tfsf<C>(p, aux, true, i0 + r, j0, ResPair4{v, v}).v);
+                res_to(x, res_tfsf_row<C>(p, aux, true, i0 + r, j0, res_from(x)));
                 put(f, x, r);
             }
         }
@@ -672,10 +717,7 @@ struct ResStrip {
         }
         if (row.xe >= 0) x_layer(px, row.b_e, row.a_e, row.i_e, dx, dbv, true, v);
         if (ye) y_layer(py_psi, true, dy, dbv, false, v);
-        if (GEN && (row.flags & RF_TFSF)) {
-            const float4 x = res_from(v);
-            res_to(v, res_tfsf<C>(p, aux, false, row.i, j0, ResPair4{x, x}).v);
-        }
+        if (GEN && (row.flags & RF_TFSF)) res_to(v, res_tfsf_row<C>(p, aux, false, row.i, j0, res_from(v)));
     }
     // fold >= 0: the step before was a sample step of the field maps, whose E partners have arrived now
     __device__ __forceinline__ void hz_h(uint32_t epoch, int64_t fold, bool update) {
@@ -753,8 +795,7 @@ struct ResStrip {
 
     __device__ __forceinline__ void hz_e(int64_t step, uint32_t epoch) {
         if (GEN && pole_mask) {
-            poles(a, 0, cx, false);
-            poles(b, 1, cy, false);
+            pole_updates(a, b);
         }
 #pragma unroll
         for (int r = 0; r < RT; ++r) {
@@ -794,15 +835,15 @@ struct ResStrip {
             }
         }
         if (GEN && pole_mask) {
-            poles(a, 0, cx, true);
-            poles(b, 1, cy, true);
+            pole_corrections(a, 0, cx);
+            pole_corrections(b, 1, cy);
         }
         if (lines) {
             sources(0, step - 1, a);
             sources(1, step - 1, b);
         }
         if (GEN && p.n_tfsf) {
-            tfsf_ab(true);
+            tfsf_ab();
         }
         mail(epoch);
         publish_hi(a);
@@ -840,8 +881,8 @@ struct ResStrip {
     }
 
     // Flux-line samples, probes and E_z maps of the state after a step.
-    __device__ __forceinline__ void samples(int64_t n) {
-        if (mons && n % p.m == 0) {
+    __device__ __forceinline__ void samples(int64_t n, bool sample) {
+        if (mons && sample) {
             const size_t s = (size_t)(n / p.m - p.q_first);
 #pragma unroll 1
             for (uint32_t left_mons = mons; left_mons; left_mons &= left_mons - 1) {
@@ -877,7 +918,7 @@ struct ResStrip {
             else get(x, b, q.ix - i0);
             q.row[n - 1] = rs_get(x, q.iy - j0);
         }
-        if (GEN && !HZ && p.n_maps && n % p.m == 0) {
+        if (GEN && !HZ && p.n_maps && sample) {
 #pragma unroll 1
             for (int r = 0; r < R; ++r) {
                 if (!(rows[r + 1].flags & RF_MAP)) continue;
@@ -969,19 +1010,22 @@ static __device__ void res_copy_psi(const Res2DJob &p, const S &s, int tid, int 
     float *base = s.pole;
     for (int k = 0; k < p.n_poles; ++k) {
         const ResPole &q = p.poles[k];
-        const int w = q.j1 - q.j0, first = max(q.i0, s.i0), n = (min(q.i1, s.i0 + s.R) - first) * w;
-        const size_t g = (size_t)(first - q.i0) * w;
+        const int wide = q.j1 - q.j0, w = res_pole_width(q, S::COLS), pad = q.j0 - q.j0 / S::COLS * S::COLS;
+        const int first = max(q.i0, s.i0), rows = max(min(q.i1, s.i0 + s.R) - first, 0), n = rows * w;
         for (int t = tid; t < n; t += nt) {
+            const int r = t / w, col = t - r * w - pad;
+            const bool in = col >= 0 && col < wide;
+            const size_t g = (size_t)(first - q.i0 + r) * wide + col;
             if (out) {
-                q.a[g + t] = base[n + t];
-                if (q.kind) q.b[g + t] = base[2 * n + t];
+                if (in) q.a[g] = base[n + t];
+                if (in && q.kind) q.b[g] = base[2 * n + t];
             } else {
-                base[t] = q.drive[g + t];
-                base[n + t] = q.a[g + t];
-                if (q.kind) base[2 * n + t] = q.b[g + t];
+                base[t] = in ? q.drive[g] : 0.0f;
+                base[n + t] = in ? q.a[g] : 0.0f;
+                if (q.kind) base[2 * n + t] = in ? q.b[g] : 0.0f;
             }
         }
-        base += res_pole_floats(q, s.i0, s.i0 + s.R);
+        base += res_pole_floats(q, s.i0, s.i0 + s.R, S::COLS);
     }
 }
 
@@ -992,14 +1036,13 @@ __host__ __device__ static inline size_t res_strip_floats(const Res2DJob &p, int
     const size_t P = (size_t)res_threads(p.ny, c) * c, R = (size_t)(i1 - i0), Y = 2 * (size_t)(p.npml + 2 * c);
     size_t n = (size_t)rt * 69 + (R + (p.da ? 2 : 0)) * P * res_coef_arrays(p) +
                ((size_t)layer_e + layer_h + 1) * P + (2 * R + 7) * Y + 16;
-    for (int k = 0; k < p.n_tfsf; ++k) n += 2 * (size_t)p.tfsf[k].aux_n;
-    for (int k = 0; k < p.n_poles; ++k) n += (size_t)res_pole_floats(p.poles[k], i0, i1);
+    for (int k = 0; k < p.n_tfsf; ++k) n += 4 * (size_t)p.tfsf[k].aux_n;
+    for (int k = 0; k < p.n_poles; ++k) n += (size_t)res_pole_floats(p.poles[k], i0, i1, c);
     return n;
 }
 
 template <bool HZ, bool GEN, int C, int RT, int NT>
 __global__ void __launch_bounds__(NT, 1) res2d_kernel(const __grid_constant__ Res2DJob job) {
-    extern __shared__ __align__(16) unsigned char res_smem[];
     __shared__ int dead_flag;
     const int tid = threadIdx.x, nt = blockDim.x;
     Res2DJob &p = *reinterpret_cast<Res2DJob *>(res_smem);
@@ -1086,8 +1129,9 @@ __global__ void __launch_bounds__(NT, 1) res2d_kernel(const __grid_constant__ Re
     __syncthreads();
     int n_e = 0, n_h = 0;
     for (int r = 0; r < s.R; ++r) n_e += s.rows[r + 1].xe >= 0, n_h += s.rows[r + 1].xh >= 0;
-    s.pole_rows = reinterpret_cast<ResPoleRows *>(s.rows + s.R + 2);
-    float *at = reinterpret_cast<float *>(s.pole_rows + p.n_poles);
+    ResPoleRows *pole_rows = reinterpret_cast<ResPoleRows *>(s.rows + s.R + 2);
+    s.pole_tab = (int)(reinterpret_cast<unsigned char *>(pole_rows) - res_smem);
+    float *at = reinterpret_cast<float *>(pole_rows + p.n_poles);
     const int P = s.P, rp = s.R * P;
     s.cx = at, at += rp;
     s.cy = at, at += HZ ? rp : 0;
@@ -1105,17 +1149,17 @@ __global__ void __launch_bounds__(NT, 1) res2d_kernel(const __grid_constant__ Re
     s.lo = at, at += RT * 34;
     s.hi = at, at += RT * 34;
     s.last = at, at += RT;
-    s.aux = at;
-    for (int k = 0; k < p.n_tfsf; ++k) at += 2 * p.tfsf[k].aux_n;
     s.pole = at;
-    for (int k = tid; k < p.n_poles; k += nt) {
+    for (int k = 0; k < p.n_poles; ++k) {
         const ResPole &q = p.poles[k];
-        float *mine = at;
-        for (int t = 0; t < k; ++t) mine += res_pole_floats(p.poles[t], s.i0, s.i0 + s.R);
-        const int first = max(q.i0, s.i0), n = max(min(q.i1, s.i0 + s.R) - first, 0) * (q.j1 - q.j0);
-        s.pole_rows[k] = ResPoleRows{mine, n, first - s.i0, q.j0, q.j1, q.kind, q.comp, q.damping, q.restoring};
+        const int first = max(q.i0, s.i0), w = res_pole_width(q, C), n = max(min(q.i1, s.i0 + s.R) - first, 0) * w;
+        if (tid == 0)
+            pole_rows[k] = ResPoleRows{(int)(at - reinterpret_cast<float *>(res_smem)), n, first - s.i0, w, q.j0 / C * C,
+                                       q.j0, q.j1, q.kind, q.damping, q.restoring, q.comp, 0};
+        at += res_pole_floats(q, s.i0, s.i0 + s.R, C);
     }
-
+    float *const aux = at;
+    s.aux = (int)(at - reinterpret_cast<float *>(res_smem));
     for (int t = tid; t < s.R * p.ny; t += nt) {
         const int r = t / p.ny, j = t - r * p.ny;
         const size_t q = (size_t)(s.i0 + r) * p.ny + j;
@@ -1169,11 +1213,15 @@ __global__ void __launch_bounds__(NT, 1) res2d_kernel(const __grid_constant__ Re
             rs_set(s.g, q, has_ghost && s.j0 + q < p.ny ? src[(size_t)ghost.i * p.ny + s.j0 + q] : 0.0f);
     }
     {
-        float *aux = s.aux;
+        float *line = aux;
         for (int k = 0; k < p.n_tfsf; ++k) {
             const ResTfsf &t = p.tfsf[k];
-            for (int q = tid; q < t.aux_n; q += nt) aux[q] = t.aux_e[q], aux[t.aux_n + q] = t.aux_h[q];
-            aux += 2 * t.aux_n;
+            const int n = t.aux_n;
+            for (int q = tid; q < n; q += nt) {
+                line[q] = t.aux_e[q], line[n + q] = t.aux_h[q];
+                line[2 * n + q] = q < n - 1 ? t.aux_coef_h[q] : 0.0f, line[3 * n + q] = t.aux_coef_e[q];
+            }
+            line += 4 * n;
         }
     }
 #pragma unroll
@@ -1221,7 +1269,7 @@ __global__ void __launch_bounds__(NT, 1) res2d_kernel(const __grid_constant__ Re
     // ---- the steps
     const bool maps = GEN && HZ && p.n_maps;
     const int64_t n_steps = p.n_steps, n0 = p.n0;
-    int64_t fold = -1;
+    int64_t fold = -1, to_sample = p.m - n0 % p.m;   // steps to the next DFT sample
     for (int64_t step = 1; step <= n_steps; ++step) {
         if constexpr (HZ) s.hz_h(epoch, fold, true);
         else s.ez_h(epoch);
@@ -1231,8 +1279,10 @@ __global__ void __launch_bounds__(NT, 1) res2d_kernel(const __grid_constant__ Re
         if constexpr (HZ) s.hz_e(step, epoch);
         else s.ez_e(step, epoch);
         if (GEN && p.n_tfsf) res_aux_e(p, s.aux, step - 1, tid, nt);
-        s.samples(n0 + step);
-        fold = maps && (n0 + step) % p.m == 0 ? n0 + step : -1;
+        const bool sample = --to_sample == 0;
+        if (sample) to_sample = p.m;
+        s.samples(n0 + step, sample);
+        fold = maps && sample ? n0 + step : -1;
         __syncthreads();
     }
     if constexpr (HZ) {
@@ -1255,11 +1305,11 @@ __global__ void __launch_bounds__(NT, 1) res2d_kernel(const __grid_constant__ Re
             }
     res_copy_psi(p, s, tid, nt, true);
     if (c == 0) {
-        const float *aux = s.aux;
+        const float *line = aux;
         for (int k = 0; k < p.n_tfsf; ++k) {
             const ResTfsf &t = p.tfsf[k];
-            for (int q = tid; q < t.aux_n; q += nt) t.aux_e[q] = aux[q], t.aux_h[q] = aux[t.aux_n + q];
-            aux += 2 * t.aux_n;
+            for (int q = tid; q < t.aux_n; q += nt) t.aux_e[q] = line[q], t.aux_h[q] = line[t.aux_n + q];
+            line += 4 * t.aux_n;
         }
     }
 }
