@@ -48,6 +48,10 @@ int os_fdtd_version(void);
  * the pooled memory.  No open_sol counterpart (open_sol relies on cupy's memory pool). */
 int os_fdtd_pool_trim(void);
 
+/* Host only: the Gaussian pulse's waveform (GaussianPulse.__call__ of a float time, open_sol/core/sources.py:40-46) at n
+ * times, in double. */
+int os_gaussian_values(double f0, double tau, double t0, const double *t, int64_t n, double *out);
+
 /* Page-locked host memory for material arrays and read-back buffers (cudaHostAlloc), so host<->device copies run at
  * full PCIe / C2C rate.  No open_sol counterpart (open_sol's cupy pool allocates device memory only). */
 int os_fdtd_host_alloc(size_t bytes, void **out);

@@ -51,6 +51,9 @@ PoolEvents *pool_events(const cudaStream_t *streams, int n);              // rec
 void pool_events_done(PoolEvents *events);                                // the releaser's reference, dropped
 int pool_trim();
 
+// Device-to-host copy behind the stream's work; dst holds the data on return.
+int read_back(void *dst, const void *src, size_t bytes, cudaStream_t stream);
+
 // A device allocation that frees itself; alloc() returns a status.
 // Grow-only: a request that fits the current capacity reuses the allocation (no free while earlier launches on the
 // stream may still read it); a larger one frees (cudaFree waits for the device) and allocates anew.  New blocks come

@@ -2353,8 +2353,8 @@ extern "C" int os_fdtd2d_read_flux_spectra(OsFdtd2D *h, int32_t monitor_id, doub
     OS_CHECK(monitor_id >= 0 && (size_t)monitor_id < h->fluxes.size(), OS_ERR_INVALID, "no flux monitor %d", monitor_id);
     OS_TRY(bind_device(h));
     FluxLine2D &f = *h->fluxes[monitor_id];
-    OS_CUDA(cudaMemcpyAsync(e_spectra, f.e_acc.ptr, f.e_acc.bytes(), cudaMemcpyDeviceToHost, h->stream));
-    OS_CUDA(cudaMemcpyAsync(h_spectra, f.h_acc.ptr, f.h_acc.bytes(), cudaMemcpyDeviceToHost, h->stream));
+    OS_TRY(read_back(e_spectra, f.e_acc.ptr, f.e_acc.bytes(), h->stream));
+    OS_TRY(read_back(h_spectra, f.h_acc.ptr, f.h_acc.bytes(), h->stream));
     OS_TRY(sync_and_check(h));
     return OS_OK;
 }
@@ -2520,7 +2520,7 @@ extern "C" int os_fdtd2d_read_dft_map(OsFdtd2D *h, int32_t map_id, float *spectr
     OS_CHECK(map_id >= 0 && (size_t)map_id < h->maps.size(), OS_ERR_INVALID, "no field-map monitor %d", map_id);
     OS_TRY(bind_device(h));
     DftMap2D &d = *h->maps[map_id];
-    OS_CUDA(cudaMemcpyAsync(spectra, d.acc.ptr, d.acc.bytes(), cudaMemcpyDeviceToHost, h->stream));
+    OS_TRY(read_back(spectra, d.acc.ptr, d.acc.bytes(), h->stream));
     OS_TRY(sync_and_check(h));
     return OS_OK;
 }
@@ -2539,7 +2539,7 @@ extern "C" int os_fdtd2d_read_field(OsFdtd2D *h, int32_t component, float *out) 
     float *src = component_ptr(h, component);
     OS_CHECK(src, OS_ERR_INVALID, "os_fdtd2d_read_field: unknown component %d", component);
     OS_TRY(bind_device(h));
-    OS_CUDA(cudaMemcpyAsync(out, src, cells(h) * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
+    OS_TRY(read_back(out, src, cells(h) * sizeof(float), h->stream));
     OS_TRY(sync_and_check(h));
     return OS_OK;
 }

@@ -858,9 +858,7 @@ extern "C" int os_fdtd3d_advance(OsFdtd3D *h, int64_t n_steps, const float *dipo
 extern "C" int os_fdtd3d_read_field(OsFdtd3D *h, int32_t component, float *out) {
     OS_CHECK(h && out && component >= 0 && component < 6, OS_ERR_INVALID, "os_fdtd3d_read_field: bad argument");
     OS_TRY(bind3(h));
-    OS_CUDA(cudaMemcpyAsync(out, fset(h, h->cur, component), h->field[component].bytes(), cudaMemcpyDeviceToHost,
-                            h->stream));
-    OS_CUDA(cudaStreamSynchronize(h->stream));
+    OS_TRY(read_back(out, fset(h, h->cur, component), h->field[component].bytes(), h->stream));
     return check_err3(h);
 }
 
@@ -879,9 +877,8 @@ extern "C" int os_fdtd3d_read_flux_pair(OsFdtd3D *h, int32_t pair_id, double *e_
     OS_TRY(bind3(h));
     const Em3DFluxPair &q = h->pairs[pair_id];
     const size_t n = 2 * (size_t)q.nf * q.n[0] * q.n[1] * q.n[2];
-    OS_CUDA(cudaMemcpyAsync(e_spectra, q.e_acc, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    OS_CUDA(cudaMemcpyAsync(h_spectra, q.h_acc, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    OS_CUDA(cudaStreamSynchronize(h->stream));
+    OS_TRY(read_back(e_spectra, q.e_acc, n * sizeof(double), h->stream));
+    OS_TRY(read_back(h_spectra, q.h_acc, n * sizeof(double), h->stream));
     return OS_OK;
 }
 

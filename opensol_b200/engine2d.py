@@ -15,7 +15,7 @@ import numpy as np
 from . import _native
 from .boundaries import build_yee_rows, face_shares
 from .constants import DTYPE, EPS0, MU0
-from .monitors import dft_phase_table
+from .monitors import dft_phase_table, step_clock
 from .poles import pole_face_sets
 
 
@@ -286,13 +286,7 @@ class FDTDEngine2D_Ez:
         side of one device chunk.  Clock: t_half = t + dt/2, t_full = t + dt accumulated in float64
         (fdtd_ez_2d.py:76-79)."""
         dt = float(self.dt)
-        t = self.time
-        t_half = np.empty(n_steps)
-        t_full = np.empty(n_steps)
-        for k in range(n_steps):
-            t_half[k] = t + 0.5 * dt
-            t = t + dt
-            t_full[k] = t
+        t_half, t_full, t = step_clock(self.time, dt, n_steps)
         rows = self._lines + self._tfsf   # line sources, then TFSF boxes (the device's value-table order)
         values = (np.stack([src.values(t_half) for src in rows]) if rows
                   else np.zeros((0, n_steps), dtype=np.float32))
@@ -332,10 +326,7 @@ class FDTDEngine2D_Ez:
         if not self._probes:
             self._step_times.extend([float('nan')] * n_steps)   # no probe reads these steps
             return
-        dt, t = float(self.dt), self.time
-        for _ in range(n_steps):
-            t = t + dt
-            self._step_times.append(t)
+        self._step_times.extend(step_clock(self.time, float(self.dt), n_steps)[1].tolist())
 
     def set_stream(self, cuda_stream):
         """Enqueue on the caller's CUDA stream (an int cudaStream_t, e.g. torch.cuda.current_stream().cuda_stream;
@@ -386,7 +377,7 @@ class FDTDEngine2D_Ez:
         h = np.empty((monitor.n_freqs, n, 2), dtype=np.float64)
         _native.check(_native.load().os_fdtd2d_read_flux_spectra(self.handle, mid, _native.dptr(e),
                                                                  _native.dptr(h)))
-        return e[..., 0] + 1j * e[..., 1], h[..., 0] + 1j * h[..., 1]
+        return e.view(np.complex128)[..., 0], h.view(np.complex128)[..., 0]
 
     def read_probe(self, probe):
         """(times float64, values float32) of a FieldProbe since it was added or the last reset."""

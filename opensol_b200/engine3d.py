@@ -19,7 +19,8 @@ from .boundaries import cpml_axis_profiles, cpml_recursion, cpml_side_rows, face
 from .constants import DTYPE
 from .domain3d import AXES
 from .material_index3d import build_material_index
-from .monitors import dft_phase_table
+from .monitors import dft_phase_table, step_clock
+from .sources import temporal_values
 
 MAX_MATERIAL_IDS = 65535
 REQUIRED_ARRAYS = ('eps_r', 'sigma_e', 'mu_r')
@@ -240,18 +241,10 @@ class FDTDEngine3D:
     def chunk_tables(self, n_steps):
         """(dipole amplitudes (n_dipoles, n_steps), first sample, n_samples, phases, clock after the chunk)."""
         dt = float(self.dt)
-        t = self.time
-        t_half = np.empty(n_steps)
-        t_full = np.empty(n_steps)
-        for k in range(n_steps):
-            t_half[k] = t + 0.5 * dt
-            t = t + dt
-            t_full[k] = t
+        t_half, t_full, t = step_clock(self.time, dt, n_steps)
         values = np.empty((len(self._dipoles), n_steps), np.float32)
         for row, (source, _) in enumerate(self._dipoles):
-            temporal = source.temporal
-            for k in range(n_steps):
-                values[row, k] = DTYPE(temporal(float(t_half[k])))
+            values[row] = temporal_values(source.temporal, t_half)
         m = self.sample_interval
         first_q = self.n_step // m + 1
         n_q = max(0, (self.n_step + n_steps) // m - first_q + 1)

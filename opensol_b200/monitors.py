@@ -47,11 +47,19 @@ def dft_sample_interval(dt, sources, monitor_frequencies, harmonic_order=1) -> i
 def dft_phase_table(omega, times, dt_m):
     """(n_samples, nf, 2) float32 table of complex64 exp(-j omega t) * dt_m per sample time (monitors.py:22-24)."""
     table = np.empty((len(times), omega.size, 2), dtype=np.float32)
-    for q, t in enumerate(times):
-        phase = -omega * float(t)
-        table[q, :, 0] = (np.cos(phase) * float(dt_m)).astype(np.float32)
-        table[q, :, 1] = (np.sin(phase) * float(dt_m)).astype(np.float32)
+    phase = -omega[None, :] * np.asarray(times, dtype=np.float64).reshape(-1, 1)
+    table[:, :, 0] = np.cos(phase) * float(dt_m)
+    table[:, :, 1] = np.sin(phase) * float(dt_m)
     return table
+
+
+def step_clock(t, dt, n_steps):
+    """(t + dt / 2, t + dt) of each of n_steps steps and the clock after them, t accumulated step by step in float64
+    (fdtd_ez_2d.py:76-79)."""
+    clock = np.full(n_steps + 1, dt, dtype=np.float64)
+    clock[0] = t
+    np.add.accumulate(clock, out=clock)
+    return clock[:-1] + 0.5 * dt, clock[1:], float(clock[-1])
 
 
 class FluxMonitor:

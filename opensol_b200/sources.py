@@ -12,6 +12,7 @@ import math
 
 import numpy as np
 
+from . import _native
 from .constants import C0, DTYPE, EPS0, ETA0, MU0
 
 
@@ -30,6 +31,14 @@ class GaussianPulse:
             return math.exp(-(delay / self.tau) ** 2) * math.sin(2.0 * math.pi * self.f0 * delay)
         delay = np.asarray(t, dtype=np.float64) - self.t0
         return np.exp(-(delay / self.tau) ** 2) * np.sin(2.0 * np.pi * self.f0 * delay)
+
+    def at(self, times):
+        """float64 values of self(float(t)) per time, by the library's loop over the same C functions."""
+        times = np.ascontiguousarray(times, dtype=np.float64)
+        out = np.empty(times.size, dtype=np.float64)
+        _native.check(_native.load().os_gaussian_values(self.f0, self.tau, self.t0, _native.dptr(times), times.size,
+                                                        _native.dptr(out)))
+        return out
 
     @property
     def duration(self) -> float:
@@ -76,6 +85,13 @@ class RickerWavelet:
 
     def spectral_limit(self) -> float:
         return 4.2 * self.f_peak
+
+
+def temporal_values(temporal, times):
+    """float64 temporal(float(t)) per time."""
+    if type(temporal) is GaussianPulse:
+        return temporal.at(times)
+    return np.array([temporal(float(t)) for t in times], dtype=np.float64)
 
 
 def make_temporal(waveform, frequency, bandwidth):
@@ -125,11 +141,8 @@ class LineSource:
 
     def values(self, t_half_list):
         """float32 amplitude * temporal(t) per time (the per-step value of LineSource.inject)."""
-        out = np.empty(len(t_half_list), dtype=np.float32)
-        temporal, amplitude = self.temporal, self.amplitude
-        for k, t in enumerate(t_half_list):
-            out[k] = DTYPE(amplitude * temporal(float(t)))
-        return out
+        # a numpy float32 times a Python float: the value is rounded to float32, then the product
+        return self.amplitude * temporal_values(self.temporal, t_half_list).astype(DTYPE)
 
 
 def sheet_admittance(line_eps, mu_r, sigma_m, omega, normal_spacing, dt):
@@ -284,7 +297,7 @@ class TFSFSource:
 
     def values(self, t_half):
         """float32 soft-source value of each step: FP32(source_scale * temporal(t + dt/2))."""
-        return np.array([DTYPE(self.source_scale * self.temporal(float(t))) for t in t_half], dtype=DTYPE)
+        return (self.source_scale * temporal_values(self.temporal, t_half)).astype(DTYPE)
 
 
 def _aux_line_terms(width, dt, half_omega_dt, index=1.0):
