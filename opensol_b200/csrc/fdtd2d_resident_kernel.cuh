@@ -344,6 +344,7 @@ struct ResStrip {
     bool end_warp, take_lo;        // the warp of column ny - 1; the thread's right neighbour comes from `lo`
     uint32_t lines, mons, probes;  // of p.lines / p.mons / p.probes, those on this thread's cells
     bool yh, ye, edge_col;
+    bool early;                    // nothing changes the thread's cells after the second phase's update
     uint32_t pole_mask;            // poles on the thread's columns
     int y_at;                      // place of the thread's columns in the rows of y-side psi and recursion
     float db_u, da_u;
@@ -367,35 +368,44 @@ struct ResStrip {
 
     __device__ __forceinline__ ResStrip(const Res2DJob &job) : p(job) {}
 
-    // The mailed values of N rows at the thread's columns (at[n] NULL: none), and one more word (extra, when extra_at).
-    // All words are loaded at once and again until every one has arrived, so a wait costs one L2 round trip and not
-    // one per word.
+    // The mailed values of N rows at the thread's columns (at[n] NULL: none), and one more word (extra_at).  peek issues
+    // the loads; take waits for them and loads all words again until every one has arrived, so a wait costs one L2 round
+    // trip and not one per word, and none when the mail was there at the peek and other work lay in between.
     template <int N>
-    __device__ __forceinline__ void receive(float2 (&v)[N][H], const uint64_t *const (&at)[N], float &extra,
-                                            const uint64_t *extra_at, uint32_t epoch) {
+    struct Mail {
+        const uint64_t *at[N], *extra_at;
+        uint64_t w[N][C], x;
+    };
+    template <int N>
+    __device__ __forceinline__ void peek(Mail<N> &m, uint32_t epoch) const {
         const uint64_t none = (uint64_t)epoch << 32;
+#pragma unroll
+        for (int n = 0; n < N; ++n)
+#pragma unroll
+            for (int c = 0; c < C; ++c) m.w[n][c] = m.at[n] && j0 + c < ny ? res_peek(m.at[n] + j0 + c) : none;
+        m.x = m.extra_at ? res_peek(m.extra_at) : none;
+    }
+    template <int N>
+    __device__ __forceinline__ void take(float2 (&v)[N][H], float &extra, Mail<N> &m, uint32_t epoch) {
         uint64_t t0 = 0;
         for (int tries = 0;; ++tries) {
-            uint64_t w[N][C], x = none;
+            bool here = (uint32_t)(m.x >> 32) == epoch;
 #pragma unroll
             for (int n = 0; n < N; ++n)
 #pragma unroll
-                for (int c = 0; c < C; ++c) w[n][c] = at[n] && j0 + c < ny ? res_peek(at[n] + j0 + c) : none;
-            if (extra_at) x = res_peek(extra_at);
-            bool here = (uint32_t)(x >> 32) == epoch;
-#pragma unroll
-            for (int n = 0; n < N; ++n)
-#pragma unroll
-                for (int c = 0; c < C; ++c) {
-                    here = here && (uint32_t)(w[n][c] >> 32) == epoch;
-                    if (c & 1) v[n][c >> 1].y = __uint_as_float((uint32_t)w[n][c]);
-                    else v[n][c >> 1].x = __uint_as_float((uint32_t)w[n][c]);
-                }
-            extra = __uint_as_float((uint32_t)x);
-            if (here) return;
+                for (int c = 0; c < C; ++c) here = here && (uint32_t)(m.w[n][c] >> 32) == epoch;
+            if (here) break;
             if (tries == 0) t0 = tb_globaltimer();
-            if ((tries & 63) == 63 && res_give_up(t0, p.err, dead)) return;
+            if ((tries & 63) == 63 && res_give_up(t0, p.err, dead)) break;
+            peek(m, epoch);
         }
+#pragma unroll
+        for (int n = 0; n < N; ++n)
+#pragma unroll
+            for (int k = 0; k < H; ++k)
+                v[n][k] = make_float2(__uint_as_float((uint32_t)m.w[n][2 * k]),
+                                      __uint_as_float((uint32_t)m.w[n][2 * k + 1]));
+        extra = __uint_as_float((uint32_t)m.x);
     }
     __device__ __forceinline__ void send(uint64_t *at, const float2 (&v)[H], uint32_t epoch) {
 #pragma unroll
@@ -406,16 +416,20 @@ struct ResStrip {
         return (size_t)(epoch & 1) * res_mail_rows(HZ) * mail_p;
     }
     // boundary rows of the present state (E_z: E_z up and down; H_z: E_x, E_y up, E_y down)
-    __device__ __forceinline__ void mail(uint32_t epoch) {
+    __device__ __forceinline__ void mail_up(uint32_t epoch) {
         uint64_t *m = to_me + slot(epoch);
-        if (has_up) {
-            send(m, HZ ? a[0] : f[0], epoch);
-            if (HZ) send(m + mail_p, b[0], epoch);
-        }
+        send(m, HZ ? a[0] : f[0], epoch);
+        if (HZ) send(m + mail_p, b[0], epoch);
+    }
+    __device__ __forceinline__ void mail_down(const float2 (&v)[H], uint32_t epoch) {
+        send(to_me + slot(epoch) + (HZ ? 2 : 1) * mail_p, v, epoch);
+    }
+    __device__ __forceinline__ void mail(uint32_t epoch) {
+        if (has_up) mail_up(epoch);
         if (has_dn) {
             float2 x[H];
             get(x, HZ ? b : f, R - 1);
-            send(m + (HZ ? 2 : 1) * mail_p, x, epoch);
+            mail_down(x, epoch);
         }
     }
 
@@ -550,6 +564,9 @@ struct ResStrip {
         if (GEN && p.da) coef(dav, da, r), coef(dbv, db, r);
     }
     __device__ __forceinline__ void ez_h(uint32_t epoch) {
+        Mail<2> mail_in{{has_up ? from_up + slot(epoch) + mail_p : nullptr, has_dn ? from_dn + slot(epoch) : nullptr},
+                        nullptr};
+        peek(mail_in, epoch);
 #pragma unroll
         for (int r = 0; r < RT; ++r) {
             if (r >= R) break;
@@ -569,12 +586,8 @@ struct ResStrip {
             if (r + 1 < RT && r + 1 < R) ez_hy(r, row, f[r], f[r + 1 < RT ? r + 1 : r], dbv, dav, xh + row.xh * P, b[r]);
         }
         float2 got[2][H];   // E_z of the row above and of the row below
-        {
-            const uint64_t *const at[2] = {has_up ? from_up + slot(epoch) + mail_p : nullptr,
-                                           has_dn ? from_dn + slot(epoch) : nullptr};
-            float none;
-            receive(got, at, none, nullptr, epoch);
-        }
+        float none;
+        take(got, none, mail_in, epoch);
         if (has_dn) {
 #pragma unroll
             for (int k = 0; k < H; ++k)
@@ -666,9 +679,11 @@ struct ResStrip {
 
     __device__ __forceinline__ void ez_e(int64_t step, uint32_t epoch) {
         if (GEN && pole_mask) pole_updates(f, f);
+        // the boundary rows first, mailed at once unless sources or corrections still change them
 #pragma unroll
-        for (int r = 0; r < RT; ++r) {
-            if (r >= R) break;
+        for (int q = 0; q < RT; ++q) {
+            const int r = q ? RT - q : 0;
+            if (r >= R) continue;
             const ResRow &row = rows[r + 1];
             float2 hl[H], cb[H], dx[H], dy[H], ca[H];
             coef(cb, cx, r);
@@ -685,6 +700,8 @@ struct ResStrip {
             }
             if (row.xe >= 0) x_layer(xe + row.xe * P, row.b_e, row.a_e, row.i_e, dx, cb, false, f[r]);
             if (ye) y_layer(yeq + r * Y, true, dy, cb, true, f[r]);
+            if (early && r == 0 && has_up) mail_up(epoch);
+            if (early && r == R - 1 && has_dn) mail_down(f[r], epoch);
         }
         if (GEN && pole_mask) pole_corrections(f, 0, cx);
         if (lines) sources(-1, step - 1, f);
@@ -698,7 +715,7 @@ struct ResStrip {
                 put(f, x, r);
             }
         }
-        mail(epoch);
+        if (!early) mail(epoch);
         publish_lo(f);
     }
 
@@ -723,10 +740,11 @@ struct ResStrip {
     __device__ __forceinline__ void hz_h(uint32_t epoch, int64_t fold, bool update) {
         const uint64_t *mu = has_up ? from_up + slot(epoch) + 2 * mail_p : nullptr, *md = from_dn + slot(epoch);
         if (GEN && fold >= 0) {
-            const uint64_t *const at[1] = {mu};
+            Mail<1> mail_up_in{{mu}, nullptr};
             float2 up[1][H];
             float none;
-            receive(up, at, none, nullptr, epoch);
+            peek(mail_up_in, epoch);
+            take(up, none, mail_up_in, epoch);
 #pragma unroll 1
             for (int r = 0; r < R; ++r) {
                 float2 h[H], x[H], xl[H], y[H], yl[H];
@@ -747,6 +765,11 @@ struct ResStrip {
             }
         }
         if (!update) return;
+        // E_y of the row above; E_x, E_y of the row below, and E_x left of the warp's first column there
+        const bool edge = has_dn && lane == 0 && j0 < ny && (j0 > 0 || py);
+        Mail<3> mail_in{{mu, has_dn ? md : nullptr, has_dn ? md + mail_p : nullptr},
+                        edge ? md + (j0 > 0 ? j0 : ny) - 1 : nullptr};
+        peek(mail_in, epoch);
 #pragma unroll
         for (int r = RT - 1; r >= 1; --r) {   // rows that need no mail
             float2 exl[H];
@@ -756,13 +779,10 @@ struct ResStrip {
                 hz_update(r, row, a[r], exl, b[r], b[r ? r - 1 : 0], xe + row.xe * P, yeq + r * Y, f[r]);
             }
         }
-        float2 got[3][H];   // E_y of the row above; E_x, E_y of the row below
+        float2 got[3][H];
         float prev_edge = 0.0f;
         {
-            const uint64_t *const at[3] = {mu, has_dn ? md : nullptr, has_dn ? md + mail_p : nullptr};
-            // E_x left of the warp's first column on the row below
-            const bool edge = has_dn && lane == 0 && j0 < ny && (j0 > 0 || py);
-            receive(got, at, prev_edge, edge ? md + (j0 > 0 ? j0 : ny) - 1 : nullptr, epoch);
+            take(got, prev_edge, mail_in, epoch);
             if (!edge) prev_edge = 0.0f;
             else if (j0 == 0) prev_edge = res_wrap_lo(prev_edge);
         }
@@ -798,8 +818,9 @@ struct ResStrip {
             pole_updates(a, b);
         }
 #pragma unroll
-        for (int r = 0; r < RT; ++r) {
-            if (r >= R) break;
+        for (int q = 0; q < RT; ++q) {   // the boundary rows first, as in ez_e
+            const int r = q ? RT - q : 0;
+            if (r >= R) continue;
             const ResRow &row = rows[r + 1];
             float2 hr[H], hd[H], cbx[H], cby[H], dx[H], dy[H], old_x[H];
             coef(cbx, cx, r);
@@ -833,6 +854,8 @@ struct ResStrip {
                 }
                 if (row.xh >= 0) x_layer(xh + row.xh * P, row.b_h, row.a_h, row.i_h, dx, cby, true, b[r]);
             }
+            if (early && r == 0 && has_up) mail_up(epoch);
+            if (early && r == R - 1 && has_dn) mail_down(b[r], epoch);
         }
         if (GEN && pole_mask) {
             pole_corrections(a, 0, cx);
@@ -845,7 +868,7 @@ struct ResStrip {
         if (GEN && p.n_tfsf) {
             tfsf_ab();
         }
-        mail(epoch);
+        if (!early) mail(epoch);
         publish_hi(a);
     }
 
@@ -1115,6 +1138,7 @@ __global__ void __launch_bounds__(NT, 1) res2d_kernel(const __grid_constant__ Re
     const int y_first = (p.ny - p.npml - 1) / C, y_hi = (p.cpml_mask >> RSY_HI) & 1 ? (p.ny - 2) / C - y_first + 1 : 0;
     s.Y = (y_lo + y_hi) * C;
     s.y_at = (tid < y_lo ? tid : y_lo + tid - y_first) * C;
+    s.early = !s.lines && !s.pole_mask && !(GEN && p.n_tfsf);
     // ---- shared memory
     s.rows = reinterpret_cast<ResRow *>(res_smem + sizeof(Res2DJob));
     for (int r = tid; r < s.R + 2; r += nt) {
@@ -1259,9 +1283,12 @@ __global__ void __launch_bounds__(NT, 1) res2d_kernel(const __grid_constant__ Re
     {
         float2 unused[2][H];
         float none;
-        const uint64_t *const at_q[2] = {s.has_up ? s.from_up + s.slot(epoch) + (HZ ? 2 : 1) * s.mail_p : nullptr,
-                                         s.has_dn ? s.from_dn + s.slot(epoch) : nullptr};
-        s.receive(unused, at_q, none, nullptr, epoch);
+        typename ResStrip<HZ, GEN, C, RT>::template Mail<2> first{
+            {s.has_up ? s.from_up + s.slot(epoch) + (HZ ? 2 : 1) * s.mail_p : nullptr,
+             s.has_dn ? s.from_dn + s.slot(epoch) : nullptr},
+            nullptr};
+        s.peek(first, epoch);
+        s.take(unused, none, first, epoch);
     }
     __syncthreads();
     if (dead_flag) return;
@@ -1320,8 +1347,8 @@ __global__ void __launch_bounds__(NT, 1) res2d_kernel(const __grid_constant__ Re
 struct ResShape {
     int c, rt, nt;
 };
-static constexpr ResShape RES_SHAPES[] = {{2, 4, 640}, {2, 8, 512},  {2, 8, 640},  {4, 4, 640}, {2, 16, 384},
-                                          {4, 8, 512}, {2, 24, 256}, {4, 10, 384}, {4, 16, 256}};
+static constexpr ResShape RES_SHAPES[] = {{2, 2, 640},  {2, 4, 640}, {2, 8, 512},  {2, 8, 640},  {4, 4, 640},
+                                          {2, 16, 384}, {4, 8, 512}, {2, 24, 256}, {4, 10, 384}, {4, 16, 256}};
 static constexpr int RES_N_SHAPES = sizeof(RES_SHAPES) / sizeof(RES_SHAPES[0]);
 
 template <bool HZ, bool GEN, int S>
