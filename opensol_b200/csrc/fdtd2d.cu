@@ -3299,8 +3299,27 @@ extern "C" int os_fdtd2d_adjoint_segment(OsAdjoint2D *a, int32_t slot, int64_t s
         a->graph_launches += 1;
         return OS_OK;
     };
-    if (n_steps == a->seg_steps) OS_TRY(run_captured(s, a->rec_graph[rb], [&] { return recompute(n_steps); }));
-    else OS_TRY(recompute(n_steps));
+    Res2DJob job{};
+    int shape = -1;
+    size_t smem = 0;
+    bool resident = false;
+    OS_TRY(resident_applies(h, job, &shape, &smem, &resident));
+    if (resident) {   // the whole segment in one launch, the box recorded by the launch (the state only: no samples)
+        ez2d_record_box_kernel<<<(unsigned)((box + 255) / 256), 256, 0, s>>>(h->ez[h->cur].ptr, h->grid.ny, a->bi0,
+                                                                              a->bi1, a->bj0, a->bj1, a->rec[rb].ptr);
+        job.n_mons = job.n_probes = 0;
+        job.rec = a->rec[rb].ptr;
+        job.rec_i0 = a->bi0, job.rec_i1 = a->bi1, job.rec_j0 = a->bj0, job.rec_j1 = a->bj1;
+        job.line_values = a->values.ptr;
+        job.values_stride = job.n_steps = n_steps;
+        job.epoch = h->res_epoch;
+        OS_TRY(launch_resident(h, job, shape, smem));
+        h->res_epoch += (uint32_t)n_steps + 1u;
+    } else if (n_steps == a->seg_steps) {
+        OS_TRY(run_captured(s, a->rec_graph[rb], [&] { return recompute(n_steps); }));
+    } else {
+        OS_TRY(recompute(n_steps));
+    }
     OS_CUDA(cudaEventRecord(a->ev_rec[rb], s));
     // ---- adjoint stream: the transposed steps backward over rec[rb], the monitor's DFT samples as sources
     OS_CUDA(cudaStreamWaitEvent(as, a->ev_rec[rb], 0));
@@ -3328,12 +3347,17 @@ extern "C" int os_fdtd2d_adjoint_segment(OsAdjoint2D *a, int32_t slot, int64_t s
         const dim3 ablock(32, 8);
         const dim3 agrid((unsigned)((h->grid.ny + 31) / 32), (unsigned)((h->grid.nx + 7) / 8));
         const float *rec = a->rec[rb].ptr;
+        q.line_normal = mon.normal_axis, q.line_position = mon.position, q.line_lo = mon.lo, q.line_n = n_line;
+        q.row_of_step = a->src_row.ptr, q.de_rows = a->src_e.ptr, q.dh_rows = a->src_h.ptr;
         int e = par;
         for (int32_t k = steps - 1; k >= 0; --k) {
-            float *lh = mon.normal_axis == 0 ? a->lhy[0].ptr : a->lhx[0].ptr;
-            ez2d_adj_source_kernel<<<(n_line + 127) / 128, 128, 0, as>>>(
-                a->le[e].ptr, lh, h->grid.ny, mon.normal_axis, mon.position, mon.lo, n_line, a->src_row.ptr, k,
-                a->src_e.ptr, a->src_h.ptr);
+            if (k == steps - 1) {   // later steps' sources are added by the H kernel of the step after them
+                float *lh = mon.normal_axis == 0 ? a->lhy[0].ptr : a->lhx[0].ptr;
+                ez2d_adj_source_kernel<<<(n_line + 127) / 128, 128, 0, as>>>(
+                    a->le[e].ptr, lh, h->grid.ny, mon.normal_axis, mon.position, mon.lo, n_line, a->src_row.ptr, k,
+                    a->src_e.ptr, a->src_h.ptr);
+            }
+            q.k_source = k - 1;
             q.le_in = a->le[e].ptr;
             q.lhx_in = a->lhx[0].ptr;
             q.lhy_in = a->lhy[0].ptr;

@@ -32,6 +32,11 @@ struct Ez2DAdjParams {
     int32_t bi0, bi1, bj0, bj1;       // design box [bi0, bi1) x [bj0, bj1)
     const float *e_next, *e_prev;     // E over the box after / before this step (box layout)
     double *grad;                     // box accumulator of lambda_E (E^{n+1} - E^n)
+    // the objective's flux line and, in the H kernel, its sources of the step before (k_source >= 0), added to the cells
+    // just written: a launch less per step than ez2d_adj_source_kernel, which only the last step of a segment needs
+    int32_t line_normal, line_position, line_lo, line_n, k_source;
+    const int32_t *row_of_step;
+    const float *de_rows, *dh_rows;
 };
 
 enum { ADJ_XLO = 0, ADJ_XHI = 1, ADJ_YLO = 2, ADJ_YHI = 3 };
@@ -164,8 +169,19 @@ __global__ void __launch_bounds__(256) ez2d_adj_h_kernel(const Ez2DAdjParams p) 
     }
     p.le_out[idx] = e;
     const float da = p.da ? p.da[idx] : p.da_u;
-    p.lhx_out[idx] = hx_updated ? da * p.lhx_in[idx] : p.lhx_in[idx];
-    p.lhy_out[idx] = hy_updated ? da * p.lhy_in[idx] : p.lhy_in[idx];
+    float hx = hx_updated ? da * p.lhx_in[idx] : p.lhx_in[idx];
+    float hy = hy_updated ? da * p.lhy_in[idx] : p.lhy_in[idx];
+    if (p.k_source >= 0 && (p.line_normal == 0 ? i : j) == p.line_position) {
+        const int c = (p.line_normal == 0 ? j : i) - p.line_lo;
+        const int row = c >= 0 && c < p.line_n ? p.row_of_step[p.k_source] : -1;
+        if (row >= 0) {
+            const size_t at = (size_t)row * p.line_n + c;
+            p.le_out[idx] += p.de_rows[at];
+            (p.line_normal == 0 ? hy : hx) += p.dh_rows[at];
+        }
+    }
+    p.lhx_out[idx] = hx;
+    p.lhy_out[idx] = hy;
 }
 
 // dJ/de and dJ/dh of the DFT sample of step k (row row_of_step[k] of de / dh, none when -1) added to lambda_E and

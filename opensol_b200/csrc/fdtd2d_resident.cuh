@@ -79,6 +79,8 @@ struct __align__(16) Res2DJob {
     ResMap maps[RES_MAX_MAPS];
     ResPole poles[RES_MAX_POLES];         // Drude poles first, each kind in add order
     ResTfsf tfsf[RES_MAX_TFSF];
+    float *rec;                           // E_z engines: E_z of a cell box after every step (step, box), or NULL
+    int32_t rec_i0, rec_i1, rec_j0, rec_j1;
     int32_t *err;
     int64_t stall_probe_ns;               // test hook of the bounded waits (0: off)
 };

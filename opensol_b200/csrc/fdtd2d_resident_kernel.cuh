@@ -344,6 +344,7 @@ struct ResStrip {
     bool end_warp, take_lo;        // the warp of column ny - 1; the thread's right neighbour comes from `lo`
     uint32_t lines, mons, probes;  // of p.lines / p.mons / p.probes, those on this thread's cells
     bool yh, ye, edge_col;
+    bool records;                  // the thread's columns reach the recorded box
     bool early;                    // nothing changes the thread's cells after the second phase's update
     uint32_t pole_mask;            // poles on the thread's columns
     int y_at;                      // place of the thread's columns in the rows of y-side psi and recursion
@@ -941,6 +942,18 @@ struct ResStrip {
             else get(x, b, q.ix - i0);
             q.row[n - 1] = rs_get(x, q.iy - j0);
         }
+        if (!HZ && records) {
+            const int w = p.rec_j1 - p.rec_j0, first = max(p.rec_i0 - i0, 0), end = min(p.rec_i1 - i0, R);
+            float *out = p.rec + (size_t)(n - p.n0) * (size_t)(p.rec_i1 - p.rec_i0) * w + (j0 - p.rec_j0);
+#pragma unroll 1
+            for (int r = first; r < end; ++r) {
+                float2 x[H];
+                get(x, f, r);
+#pragma unroll
+                for (int c = 0; c < C; ++c)
+                    if (j0 + c >= p.rec_j0 && j0 + c < p.rec_j1) out[(i0 + r - p.rec_i0) * w + c] = rs_get(x, c);
+            }
+        }
         if (GEN && !HZ && p.n_maps && sample) {
 #pragma unroll 1
             for (int r = 0; r < R; ++r) {
@@ -1138,6 +1151,7 @@ __global__ void __launch_bounds__(NT, 1) res2d_kernel(const __grid_constant__ Re
     const int y_first = (p.ny - p.npml - 1) / C, y_hi = (p.cpml_mask >> RSY_HI) & 1 ? (p.ny - 2) / C - y_first + 1 : 0;
     s.Y = (y_lo + y_hi) * C;
     s.y_at = (tid < y_lo ? tid : y_lo + tid - y_first) * C;
+    s.records = !HZ && p.rec && p.rec_j0 < s.j0 + C && p.rec_j1 > s.j0;
     s.early = !s.lines && !s.pole_mask && !(GEN && p.n_tfsf);
     // ---- shared memory
     s.rows = reinterpret_cast<ResRow *>(res_smem + sizeof(Res2DJob));
