@@ -1894,7 +1894,7 @@ static Res2DJob resident_job(const OsFdtd2D *h) {
 
 // Whether the handle's chunks run in the resident form now (job, shape and smem filled), planning its strips on the
 // first call.  It takes every feature of the per-step kernels within the parameter block's limits, on any grid whose
-// strips fit a kernel shape (registers: about 2 M cells) and a multiprocessor's shared memory; stream capture keeps the
+// strips fit a kernel shape (registers: 1.3 to 2 M cells) and a multiprocessor's shared memory; stream capture keeps the
 // launch-per-step forms, whose work a captured graph may replay beside other kernels.
 static int resident_applies(OsFdtd2D *h, Res2DJob &job, int *shape, size_t *smem, bool *yes) {
     *yes = false;
@@ -1903,11 +1903,15 @@ static int resident_applies(OsFdtd2D *h, Res2DJob &job, int *shape, size_t *smem
     if (h->lines.size() > RES_MAX_LINES || h->fluxes.size() > RES_MAX_MONS || h->maps.size() > RES_MAX_MAPS ||
         h->poles.size() > RES_MAX_POLES || h->tfsf.size() > RES_MAX_TFSF)
         return OS_OK;
-    if (res2d_shape(g.ny, (g.nx + h->sm_count - 1) / h->sm_count) < 0) return OS_OK;
+    const bool blocked = h->poles.empty() && h->tfsf.empty();   // the alternative: blocked, or launches per half step
+    if (res2d_shape(g.ny, (g.nx + h->sm_count - 1) / h->sm_count, blocked) < 0) return OS_OK;
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     OS_CUDA(cudaStreamIsCapturing(h->stream, &capture));
     if (capture != cudaStreamCaptureStatusNone) return OS_OK;
     if (h->res_rows.empty()) {
+        int cooperative = 0;
+        OS_CUDA(cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, h->device));
+        if (!cooperative) return OS_OK;
         h->res_rows = resident_strips(h);
         OS_CUDA(cudaDeviceGetAttribute(&h->res_smem_limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
         h->res_smem_limit -= 1024;   // the kernel's own static shared memory
@@ -1915,7 +1919,7 @@ static int resident_applies(OsFdtd2D *h, Res2DJob &job, int *shape, size_t *smem
     int max_rows = 0;
     for (size_t c = 0; c + 1 < h->res_rows.size(); ++c)
         max_rows = std::max(max_rows, h->res_rows[c + 1] - h->res_rows[c]);
-    *shape = res2d_shape(g.ny, max_rows);
+    *shape = res2d_shape(g.ny, max_rows, blocked);
     if (*shape < 0) return OS_OK;
     job = resident_job(h);
     const bool lo = g.cpml_sides & 1, hi = g.cpml_sides & 2;

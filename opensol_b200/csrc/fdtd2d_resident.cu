@@ -6,9 +6,11 @@ cudaError_t res2d_launch_ez_gen(int shape, const Res2DJob &job, size_t smem, cud
 cudaError_t res2d_launch_hz_plain(int shape, const Res2DJob &job, size_t smem, cudaStream_t stream);
 cudaError_t res2d_launch_hz_gen(int shape, const Res2DJob &job, size_t smem, cudaStream_t stream);
 
-int res2d_shape(int ny, int max_rows) {
+int res2d_shape(int ny, int max_rows, bool blocked_takes_it) {
     for (int s = 0; s < RES_N_SHAPES; ++s)
-        if (max_rows <= RES_SHAPES[s].rt && (ny + RES_SHAPES[s].c - 1) / RES_SHAPES[s].c <= RES_SHAPES[s].nt) return s;
+        if (!(blocked_takes_it && RES_SHAPES[s].blocked_is_faster) && max_rows <= RES_SHAPES[s].rt &&
+            (ny + RES_SHAPES[s].c - 1) / RES_SHAPES[s].c <= RES_SHAPES[s].nt)
+            return s;
     return -1;
 }
 

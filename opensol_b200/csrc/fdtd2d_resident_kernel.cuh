@@ -19,8 +19,8 @@
 //
 // What bounds it: small strips (240 x 120 cells) wait for the mail, about 1 us from store to poll across L2, plus two
 // block barriers; large ones (1075 x 1075) the issue rate of the row updates.  Measured on a B200, device time per step
-// against the launches per step before it: 270 x 120 cells 2.0 us (15), 441 x 393 lossy 3.6 us (20), 1075 x 1075 6.1 us
-// (17), 924 x 724 H_z 4.9 us (18).  Fields in shared memory instead of registers (one cell at a time) took 18 us at
+// against the launches per step before it: 270 x 120 cells 1.9 us (15), 441 x 393 lossy 3.4 us (20), 1075 x 1075 6.1 us
+// (17), 930 x 730 H_z 4.6 us (18).  Fields in shared memory instead of registers (one cell at a time) took 18 us at
 // 1075 x 1075; so did polling one mailed word after the other (an L2 round trip each).
 //
 // GEN adds what plain lossless runs do not need: ca / da / db words, field maps, poles, plane-wave boxes.
@@ -1358,23 +1358,34 @@ __global__ void __launch_bounds__(NT, 1) res2d_kernel(const __grid_constant__ Re
 // The kernels' shapes: C columns a thread, up to RT rows a strip, up to NT threads, in order of preference (fewest
 // registers first).  The register file bounds them: NT threads have 65,536 / NT registers each (in steps of 128
 // threads: 96 at 640, 128 at 512, 168 at 384, 255 at 256), of which 3 C RT hold fields and about 45 the rest.
+// Four columns a thread run at about half the rate of two (fewer warps, spills), so past 6 rows of them the blocked
+// kernels are faster and only runs that those do not take (poles, plane-wave boxes: about 50 us a step in launches per
+// half step) use the shape.  Measured, us per step here and blocked, E_z / H_z: 1110 x 1130 7.2, 15.6 / 8.4, 18.9; 530 x
+// 1980 9.1, 13.0 / 12.6, 12.9; 830 x 1430 12.6, 14.4 / 15.1, 17.8; 3430 x 330 14.1, 15.2 / 14.0, 16.9; with four columns
+// and 8 to 16 rows 1130 x 1430 15.3, 14.4 and 1730 x 980 18.1, 13.0.
 struct ResShape {
     int c, rt, nt;
+    bool blocked_is_faster;
 };
-static constexpr ResShape RES_SHAPES[] = {{2, 2, 640},  {2, 4, 640}, {2, 8, 512},  {2, 8, 640},  {4, 4, 640},
-                                          {2, 16, 384}, {4, 8, 512}, {2, 24, 256}, {4, 10, 384}, {4, 16, 256}};
+static constexpr ResShape RES_SHAPES[] = {
+    {2, 2, 640, false}, {2, 4, 640, false},  {2, 8, 512, false}, {2, 8, 640, false},  {4, 4, 640, false},
+    {2, 16, 384, false}, {4, 6, 512, false}, {2, 24, 256, false}, {4, 10, 384, true}, {4, 16, 256, true}};
 static constexpr int RES_N_SHAPES = sizeof(RES_SHAPES) / sizeof(RES_SHAPES[0]);
 
-template <bool HZ, bool GEN, int S>
-static cudaError_t res_launch_shape(const Res2DJob &job, size_t smem, cudaStream_t stream) {
-    constexpr ResShape sh = RES_SHAPES[S];
-    auto kernel = res2d_kernel<HZ, GEN, sh.c, sh.rt, sh.nt>;
+template <bool HZ, bool GEN, int C, int RT, int NT>
+static cudaError_t res_launch_kernel(const Res2DJob &job, size_t smem, cudaStream_t stream) {
+    auto kernel = res2d_kernel<HZ, GEN, C, RT, NT>;
     cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return err;
     void *args[] = {const_cast<Res2DJob *>(&job)};
-    const int threads = res_threads(job.ny, sh.c);
-    return cudaLaunchCooperativeKernel((const void *)kernel, dim3((unsigned)job.n_cta), dim3((unsigned)threads), args,
-                                       smem, stream);
+    return cudaLaunchCooperativeKernel((const void *)kernel, dim3((unsigned)job.n_cta),
+                                       dim3((unsigned)res_threads(job.ny, C)), args, smem, stream);
+}
+template <bool HZ, bool GEN, int S>
+static cudaError_t res_launch_shape(const Res2DJob &job, size_t smem, cudaStream_t stream) {
+    constexpr ResShape sh = RES_SHAPES[S];
+    if constexpr (!GEN && sh.blocked_is_faster) return cudaErrorInvalidValue;   // plain runs never ask for it
+    else return res_launch_kernel<HZ, GEN, sh.c, sh.rt, sh.nt>(job, smem, stream);
 }
 template <bool HZ, bool GEN, int S = 0>
 static cudaError_t res_launch_any(int shape, const Res2DJob &job, size_t smem, cudaStream_t stream) {

@@ -116,6 +116,21 @@ def test_resident_among_the_other_forms(pol):
     _compare(dict(pol=pol, nx=200, ny=164, boundaries='pml', npml=10, seed=7, maps=(3,), probes=2), (20, 31, 25), 1)
 
 
+def test_resident_chunk_past_the_staged_samples():
+    """A chunk with more DFT samples than one launch stages (every step sampled) runs in several launches."""
+    got = []
+    for variant in (3, 0):
+        sim, out = _sim('ez', 30, 1500, 'pml', 10, seed=9)
+        sim.em.engine.configure(variant=variant)
+        sim.em.engine.set_sample_interval(1)
+        sim.em.engine.advance(3000)
+        if variant == 3:
+            assert sim.em.engine.launch_count() == 2 * (1 + 3)
+        got.append(_outputs(sim, out))
+    for a, b in zip(*got):
+        np.testing.assert_array_equal(a, b)
+
+
 def test_resident_two_rows():
     """The smallest strips: a periodic grid of 2 x 40 cells, and of 3 rows."""
     for nx in (2, 3):
