@@ -19,8 +19,8 @@
 //
 // What bounds it: small strips (240 x 120 cells) wait for the mail, about 1 us from store to poll across L2, plus two
 // block barriers; large ones (1075 x 1075) the issue rate of the row updates.  Measured on a B200, device time per step
-// against the launches per step before it: 270 x 120 cells 1.9 us (15), 441 x 393 lossy 3.4 us (20), 1075 x 1075 6.1 us
-// (17), 930 x 730 H_z 4.6 us (18).  Fields in shared memory instead of registers (one cell at a time) took 18 us at
+// against the launches per step before it: 270 x 120 cells 2.0 us (15), 441 x 393 lossy 3.6 us (20), 1075 x 1075 6.1 us
+// (17), 930 x 730 H_z 4.9 us (18).  Fields in shared memory instead of registers (one cell at a time) took 18 us at
 // 1075 x 1075; so did polling one mailed word after the other (an L2 round trip each).
 //
 // GEN adds what plain lossless runs do not need: ca / da / db words, field maps, poles, plane-wave boxes.
@@ -345,7 +345,6 @@ struct ResStrip {
     uint32_t lines, mons, probes;  // of p.lines / p.mons / p.probes, those on this thread's cells
     bool yh, ye, edge_col;
     bool records;                  // the thread's columns reach the recorded box
-    bool early;                    // nothing changes the thread's cells after the second phase's update
     uint32_t pole_mask;            // poles on the thread's columns
     int y_at;                      // place of the thread's columns in the rows of y-side psi and recursion
     float db_u, da_u;
@@ -369,44 +368,35 @@ struct ResStrip {
 
     __device__ __forceinline__ ResStrip(const Res2DJob &job) : p(job) {}
 
-    // The mailed values of N rows at the thread's columns (at[n] NULL: none), and one more word (extra_at).  peek issues
-    // the loads; take waits for them and loads all words again until every one has arrived, so a wait costs one L2 round
-    // trip and not one per word, and none when the mail was there at the peek and other work lay in between.
+    // The mailed values of N rows at the thread's columns (at[n] NULL: none), and one more word (extra, when extra_at).
+    // All words are loaded at once and again until every one has arrived, so a wait costs one L2 round trip and not
+    // one per word.
     template <int N>
-    struct Mail {
-        const uint64_t *at[N], *extra_at;
-        uint64_t w[N][C], x;
-    };
-    template <int N>
-    __device__ __forceinline__ void peek(Mail<N> &m, uint32_t epoch) const {
+    __device__ __forceinline__ void receive(float2 (&v)[N][H], const uint64_t *const (&at)[N], float &extra,
+                                            const uint64_t *extra_at, uint32_t epoch) {
         const uint64_t none = (uint64_t)epoch << 32;
-#pragma unroll
-        for (int n = 0; n < N; ++n)
-#pragma unroll
-            for (int c = 0; c < C; ++c) m.w[n][c] = m.at[n] && j0 + c < ny ? res_peek(m.at[n] + j0 + c) : none;
-        m.x = m.extra_at ? res_peek(m.extra_at) : none;
-    }
-    template <int N>
-    __device__ __forceinline__ void take(float2 (&v)[N][H], float &extra, Mail<N> &m, uint32_t epoch) {
         uint64_t t0 = 0;
         for (int tries = 0;; ++tries) {
-            bool here = (uint32_t)(m.x >> 32) == epoch;
+            uint64_t w[N][C], x = none;
 #pragma unroll
             for (int n = 0; n < N; ++n)
 #pragma unroll
-                for (int c = 0; c < C; ++c) here = here && (uint32_t)(m.w[n][c] >> 32) == epoch;
-            if (here) break;
+                for (int c = 0; c < C; ++c) w[n][c] = at[n] && j0 + c < ny ? res_peek(at[n] + j0 + c) : none;
+            if (extra_at) x = res_peek(extra_at);
+            bool here = (uint32_t)(x >> 32) == epoch;
+#pragma unroll
+            for (int n = 0; n < N; ++n)
+#pragma unroll
+                for (int c = 0; c < C; ++c) {
+                    here = here && (uint32_t)(w[n][c] >> 32) == epoch;
+                    if (c & 1) v[n][c >> 1].y = __uint_as_float((uint32_t)w[n][c]);
+                    else v[n][c >> 1].x = __uint_as_float((uint32_t)w[n][c]);
+                }
+            extra = __uint_as_float((uint32_t)x);
+            if (here) return;
             if (tries == 0) t0 = tb_globaltimer();
-            if ((tries & 63) == 63 && res_give_up(t0, p.err, dead)) break;
-            peek(m, epoch);
+            if ((tries & 63) == 63 && res_give_up(t0, p.err, dead)) return;
         }
-#pragma unroll
-        for (int n = 0; n < N; ++n)
-#pragma unroll
-            for (int k = 0; k < H; ++k)
-                v[n][k] = make_float2(__uint_as_float((uint32_t)m.w[n][2 * k]),
-                                      __uint_as_float((uint32_t)m.w[n][2 * k + 1]));
-        extra = __uint_as_float((uint32_t)m.x);
     }
     __device__ __forceinline__ void send(uint64_t *at, const float2 (&v)[H], uint32_t epoch) {
 #pragma unroll
@@ -417,20 +407,16 @@ struct ResStrip {
         return (size_t)(epoch & 1) * res_mail_rows(HZ) * mail_p;
     }
     // boundary rows of the present state (E_z: E_z up and down; H_z: E_x, E_y up, E_y down)
-    __device__ __forceinline__ void mail_up(uint32_t epoch) {
-        uint64_t *m = to_me + slot(epoch);
-        send(m, HZ ? a[0] : f[0], epoch);
-        if (HZ) send(m + mail_p, b[0], epoch);
-    }
-    __device__ __forceinline__ void mail_down(const float2 (&v)[H], uint32_t epoch) {
-        send(to_me + slot(epoch) + (HZ ? 2 : 1) * mail_p, v, epoch);
-    }
     __device__ __forceinline__ void mail(uint32_t epoch) {
-        if (has_up) mail_up(epoch);
+        uint64_t *m = to_me + slot(epoch);
+        if (has_up) {
+            send(m, HZ ? a[0] : f[0], epoch);
+            if (HZ) send(m + mail_p, b[0], epoch);
+        }
         if (has_dn) {
             float2 x[H];
             get(x, HZ ? b : f, R - 1);
-            mail_down(x, epoch);
+            send(m + (HZ ? 2 : 1) * mail_p, x, epoch);
         }
     }
 
@@ -565,9 +551,6 @@ struct ResStrip {
         if (GEN && p.da) coef(dav, da, r), coef(dbv, db, r);
     }
     __device__ __forceinline__ void ez_h(uint32_t epoch) {
-        Mail<2> mail_in{{has_up ? from_up + slot(epoch) + mail_p : nullptr, has_dn ? from_dn + slot(epoch) : nullptr},
-                        nullptr};
-        peek(mail_in, epoch);
 #pragma unroll
         for (int r = 0; r < RT; ++r) {
             if (r >= R) break;
@@ -587,8 +570,12 @@ struct ResStrip {
             if (r + 1 < RT && r + 1 < R) ez_hy(r, row, f[r], f[r + 1 < RT ? r + 1 : r], dbv, dav, xh + row.xh * P, b[r]);
         }
         float2 got[2][H];   // E_z of the row above and of the row below
-        float none;
-        take(got, none, mail_in, epoch);
+        {
+            const uint64_t *const at[2] = {has_up ? from_up + slot(epoch) + mail_p : nullptr,
+                                           has_dn ? from_dn + slot(epoch) : nullptr};
+            float none;
+            receive(got, at, none, nullptr, epoch);
+        }
         if (has_dn) {
 #pragma unroll
             for (int k = 0; k < H; ++k)
@@ -680,11 +667,9 @@ struct ResStrip {
 
     __device__ __forceinline__ void ez_e(int64_t step, uint32_t epoch) {
         if (GEN && pole_mask) pole_updates(f, f);
-        // the boundary rows first, mailed at once unless sources or corrections still change them
 #pragma unroll
-        for (int q = 0; q < RT; ++q) {
-            const int r = q ? RT - q : 0;
-            if (r >= R) continue;
+        for (int r = 0; r < RT; ++r) {
+            if (r >= R) break;
             const ResRow &row = rows[r + 1];
             float2 hl[H], cb[H], dx[H], dy[H], ca[H];
             coef(cb, cx, r);
@@ -701,8 +686,6 @@ struct ResStrip {
             }
             if (row.xe >= 0) x_layer(xe + row.xe * P, row.b_e, row.a_e, row.i_e, dx, cb, false, f[r]);
             if (ye) y_layer(yeq + r * Y, true, dy, cb, true, f[r]);
-            if (early && r == 0 && has_up) mail_up(epoch);
-            if (early && r == R - 1 && has_dn) mail_down(f[r], epoch);
         }
         if (GEN && pole_mask) pole_corrections(f, 0, cx);
         if (lines) sources(-1, step - 1, f);
@@ -716,7 +699,7 @@ struct ResStrip {
                 put(f, x, r);
             }
         }
-        if (!early) mail(epoch);
+        mail(epoch);
         publish_lo(f);
     }
 
@@ -741,11 +724,10 @@ struct ResStrip {
     __device__ __forceinline__ void hz_h(uint32_t epoch, int64_t fold, bool update) {
         const uint64_t *mu = has_up ? from_up + slot(epoch) + 2 * mail_p : nullptr, *md = from_dn + slot(epoch);
         if (GEN && fold >= 0) {
-            Mail<1> mail_up_in{{mu}, nullptr};
+            const uint64_t *const at[1] = {mu};
             float2 up[1][H];
             float none;
-            peek(mail_up_in, epoch);
-            take(up, none, mail_up_in, epoch);
+            receive(up, at, none, nullptr, epoch);
 #pragma unroll 1
             for (int r = 0; r < R; ++r) {
                 float2 h[H], x[H], xl[H], y[H], yl[H];
@@ -766,11 +748,6 @@ struct ResStrip {
             }
         }
         if (!update) return;
-        // E_y of the row above; E_x, E_y of the row below, and E_x left of the warp's first column there
-        const bool edge = has_dn && lane == 0 && j0 < ny && (j0 > 0 || py);
-        Mail<3> mail_in{{mu, has_dn ? md : nullptr, has_dn ? md + mail_p : nullptr},
-                        edge ? md + (j0 > 0 ? j0 : ny) - 1 : nullptr};
-        peek(mail_in, epoch);
 #pragma unroll
         for (int r = RT - 1; r >= 1; --r) {   // rows that need no mail
             float2 exl[H];
@@ -780,10 +757,13 @@ struct ResStrip {
                 hz_update(r, row, a[r], exl, b[r], b[r ? r - 1 : 0], xe + row.xe * P, yeq + r * Y, f[r]);
             }
         }
-        float2 got[3][H];
+        float2 got[3][H];   // E_y of the row above; E_x, E_y of the row below
         float prev_edge = 0.0f;
         {
-            take(got, prev_edge, mail_in, epoch);
+            const uint64_t *const at[3] = {mu, has_dn ? md : nullptr, has_dn ? md + mail_p : nullptr};
+            // E_x left of the warp's first column on the row below
+            const bool edge = has_dn && lane == 0 && j0 < ny && (j0 > 0 || py);
+            receive(got, at, prev_edge, edge ? md + (j0 > 0 ? j0 : ny) - 1 : nullptr, epoch);
             if (!edge) prev_edge = 0.0f;
             else if (j0 == 0) prev_edge = res_wrap_lo(prev_edge);
         }
@@ -819,9 +799,8 @@ struct ResStrip {
             pole_updates(a, b);
         }
 #pragma unroll
-        for (int q = 0; q < RT; ++q) {   // the boundary rows first, as in ez_e
-            const int r = q ? RT - q : 0;
-            if (r >= R) continue;
+        for (int r = 0; r < RT; ++r) {
+            if (r >= R) break;
             const ResRow &row = rows[r + 1];
             float2 hr[H], hd[H], cbx[H], cby[H], dx[H], dy[H], old_x[H];
             coef(cbx, cx, r);
@@ -855,8 +834,6 @@ struct ResStrip {
                 }
                 if (row.xh >= 0) x_layer(xh + row.xh * P, row.b_h, row.a_h, row.i_h, dx, cby, true, b[r]);
             }
-            if (early && r == 0 && has_up) mail_up(epoch);
-            if (early && r == R - 1 && has_dn) mail_down(b[r], epoch);
         }
         if (GEN && pole_mask) {
             pole_corrections(a, 0, cx);
@@ -869,7 +846,7 @@ struct ResStrip {
         if (GEN && p.n_tfsf) {
             tfsf_ab();
         }
-        if (!early) mail(epoch);
+        mail(epoch);
         publish_hi(a);
     }
 
@@ -1152,7 +1129,6 @@ __global__ void __launch_bounds__(NT, 1) res2d_kernel(const __grid_constant__ Re
     s.Y = (y_lo + y_hi) * C;
     s.y_at = (tid < y_lo ? tid : y_lo + tid - y_first) * C;
     s.records = !HZ && p.rec && p.rec_j0 < s.j0 + C && p.rec_j1 > s.j0;
-    s.early = !s.lines && !s.pole_mask && !(GEN && p.n_tfsf);
     // ---- shared memory
     s.rows = reinterpret_cast<ResRow *>(res_smem + sizeof(Res2DJob));
     for (int r = tid; r < s.R + 2; r += nt) {
@@ -1297,12 +1273,9 @@ __global__ void __launch_bounds__(NT, 1) res2d_kernel(const __grid_constant__ Re
     {
         float2 unused[2][H];
         float none;
-        typename ResStrip<HZ, GEN, C, RT>::template Mail<2> first{
-            {s.has_up ? s.from_up + s.slot(epoch) + (HZ ? 2 : 1) * s.mail_p : nullptr,
-             s.has_dn ? s.from_dn + s.slot(epoch) : nullptr},
-            nullptr};
-        s.peek(first, epoch);
-        s.take(unused, none, first, epoch);
+        const uint64_t *const at_q[2] = {s.has_up ? s.from_up + s.slot(epoch) + (HZ ? 2 : 1) * s.mail_p : nullptr,
+                                         s.has_dn ? s.from_dn + s.slot(epoch) : nullptr};
+        s.receive(unused, at_q, none, nullptr, epoch);
     }
     __syncthreads();
     if (dead_flag) return;
@@ -1358,8 +1331,8 @@ __global__ void __launch_bounds__(NT, 1) res2d_kernel(const __grid_constant__ Re
 // The kernels' shapes: C columns a thread, up to RT rows a strip, up to NT threads, in order of preference (fewest
 // registers first).  The register file bounds them: NT threads have 65,536 / NT registers each (in steps of 128
 // threads: 96 at 640, 128 at 512, 168 at 384, 255 at 256), of which 3 C RT hold fields and about 45 the rest.
-// Four columns a thread run at about half the rate of two (fewer warps, spills), so past 6 rows of them the blocked
-// kernels are faster and only runs that those do not take (poles, plane-wave boxes: about 50 us a step in launches per
+// Four columns a thread run at about half the rate of two (fewer warps, spills): little or nothing faster than the
+// blocked kernels, so only runs that those do not take (poles, plane-wave boxes: about 50 us a step in launches per
 // half step) use the shape.  Measured, us per step here and blocked, E_z / H_z: 1110 x 1130 7.2, 15.6 / 8.4, 18.9; 530 x
 // 1980 9.1, 13.0 / 12.6, 12.9; 830 x 1430 12.6, 14.4 / 15.1, 17.8; 3430 x 330 14.1, 15.2 / 14.0, 16.9; with four columns
 // and 8 to 16 rows 1130 x 1430 15.3, 14.4 and 1730 x 980 18.1, 13.0.
@@ -1368,8 +1341,8 @@ struct ResShape {
     bool blocked_is_faster;
 };
 static constexpr ResShape RES_SHAPES[] = {
-    {2, 2, 640, false}, {2, 4, 640, false},  {2, 8, 512, false}, {2, 8, 640, false},  {4, 4, 640, false},
-    {2, 16, 384, false}, {4, 6, 512, false}, {2, 24, 256, false}, {4, 10, 384, true}, {4, 16, 256, true}};
+    {2, 4, 640, false}, {2, 8, 512, false}, {2, 8, 640, false}, {4, 4, 640, true},  {2, 16, 384, false},
+    {4, 8, 512, true},  {2, 24, 256, false}, {4, 10, 384, true}, {4, 16, 256, true}};
 static constexpr int RES_N_SHAPES = sizeof(RES_SHAPES) / sizeof(RES_SHAPES[0]);
 
 template <bool HZ, bool GEN, int C, int RT, int NT>
