@@ -120,10 +120,10 @@ def test_resident_chunk_past_the_staged_samples():
     """A chunk with more DFT samples than one launch stages (every step sampled) runs in several launches."""
     got = []
     for variant in (3, 0):
-        sim, out = _sim('ez', 30, 1500, 'pml', 10, seed=9)
+        sim, out = _sim('ez', 30, 1200, 'pml', 10, seed=9)
         sim.em.engine.configure(variant=variant)
         sim.em.engine.set_sample_interval(1)
-        sim.em.engine.advance(3000)
+        sim.em.engine.advance(4000)
         if variant == 3:
             assert sim.em.engine.launch_count() == 2 * (1 + 3)
         got.append(_outputs(sim, out))
