@@ -3065,7 +3065,11 @@ struct OsAdjoint2D {
     cudaStream_t adj_stream = nullptr;
     cudaEvent_t ev_rec[2] = {nullptr, nullptr}, ev_swept[2] = {nullptr, nullptr};
     bool swept_pending[2] = {false, false};
-    cudaGraphExec_t rec_graph[2] = {nullptr, nullptr};           // full-length recomputation, per rec buffer
+    // full-length recomputation, per rec buffer and field set (a forward run of an odd number of launches leaves the other
+    // set current, and a checkpoint is restored into the current one), with the arguments each was captured with
+    cudaGraphExec_t rec_graph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
+    Ez2DParams rec_params[2][2];
+    const float *rec_values[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
     cudaGraphExec_t sweep_graph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};   // per rec buffer and parity
     int sweep_monitor[2][2] = {{-1, -1}, {-1, -1}};
     int64_t graph_launches = 0;
@@ -3183,7 +3187,8 @@ extern "C" int os_fdtd2d_adjoint_destroy(OsAdjoint2D *a) {
     cudaStreamSynchronize(a->h->stream);
     if (a->adj_stream) cudaStreamSynchronize(a->adj_stream);
     for (int b = 0; b < 2; ++b) {
-        if (a->rec_graph[b]) cudaGraphExecDestroy(a->rec_graph[b]);
+        for (cudaGraphExec_t g : a->rec_graph[b])
+            if (g) cudaGraphExecDestroy(g);
         for (cudaGraphExec_t g : a->sweep_graph[b])
             if (g) cudaGraphExecDestroy(g);
         if (a->ev_rec[b]) cudaEventDestroy(a->ev_rec[b]);
@@ -3283,7 +3288,7 @@ extern "C" int os_fdtd2d_adjoint_segment(OsAdjoint2D *a, int32_t slot, int64_t s
         }
         return OS_OK;
     };
-    // a full-length segment replays a captured graph (its arguments are the same for every segment using rec[rb])
+    // a full-length segment replays a captured graph while its arguments are those of the capture
     auto run_captured = [&](cudaStream_t stream, cudaGraphExec_t &exec, const std::function<int()> &body) -> int {
         if (!exec) {
             cudaGraph_t g = nullptr;
@@ -3320,7 +3325,16 @@ extern "C" int os_fdtd2d_adjoint_segment(OsAdjoint2D *a, int32_t slot, int64_t s
         OS_TRY(launch_resident(h, job, shape, smem));
         h->res_epoch += (uint32_t)n_steps + 1u;
     } else if (n_steps == a->seg_steps) {
-        OS_TRY(run_captured(s, a->rec_graph[rb], [&] { return recompute(n_steps); }));
+        const int c = h->cur;
+        const Ez2DParams now = make_params(h);
+        cudaGraphExec_t &exec = a->rec_graph[rb][c];
+        if (exec && (memcmp(&now, &a->rec_params[rb][c], sizeof now) || a->values.ptr != a->rec_values[rb][c])) {
+            OS_CUDA(cudaGraphExecDestroy(exec));
+            exec = nullptr;
+        }
+        memcpy(&a->rec_params[rb][c], &now, sizeof now);
+        a->rec_values[rb][c] = a->values.ptr;
+        OS_TRY(run_captured(s, exec, [&] { return recompute(n_steps); }));
     } else {
         OS_TRY(recompute(n_steps));
     }

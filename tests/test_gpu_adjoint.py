@@ -75,6 +75,23 @@ def test_adjoint_gradient_against_oracle_adjoint_and_fd():
     adj.close()
 
 
+@pytest.mark.parametrize('variant', [1, 3])
+@pytest.mark.parametrize('n_steps', range(395, 401))
+def test_every_gradient_of_one_object(variant, n_steps):
+    """Passes on one object give one gradient, whichever of the two field sets a forward run ends in: the lengths take
+    odd and even numbers of blocked launches, and the recomputation's captured launches belong to one set."""
+    eps = _eps_box()
+    sim, mon = _product(eps)
+    sim.em.engine.configure(variant=variant)
+    adj = FluxAdjoint2D(sim, mon, 0, BOX, n_steps, checkpoint_every=64)
+    J = adj.forward(eps)
+    g = adj.backward()
+    for _ in range(3):
+        assert adj.forward(eps) == J
+        np.testing.assert_array_equal(adj.backward(), g)
+    adj.close()
+
+
 def test_torch_autograd_function():
     import torch
     eps = _eps_box()
