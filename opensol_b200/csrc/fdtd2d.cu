@@ -3313,10 +3313,11 @@ extern "C" int os_fdtd2d_adjoint_segment(OsAdjoint2D *a, int32_t slot, int64_t s
     size_t smem = 0;
     bool resident = false;
     OS_TRY(resident_applies(h, job, &shape, &smem, &resident));
-    if (resident) {   // the whole segment in one launch, the box recorded by the launch (the state only: no samples)
+    if (resident) {   // the whole segment in one launch, the box recorded by the launch (the state only: no samples, for
+                      // which it has no tables: flux lines, probes and field maps keep the forward run's)
         ez2d_record_box_kernel<<<(unsigned)((box + 255) / 256), 256, 0, s>>>(h->ez[h->cur].ptr, h->grid.ny, a->bi0,
                                                                               a->bi1, a->bj0, a->bj1, a->rec[rb].ptr);
-        job.n_mons = job.n_probes = 0;
+        job.n_mons = job.n_probes = job.n_maps = 0;
         job.rec = a->rec[rb].ptr;
         job.rec_i0 = a->bi0, job.rec_i1 = a->bi1, job.rec_j0 = a->bj0, job.rec_j1 = a->bj1;
         job.line_values = a->values.ptr;

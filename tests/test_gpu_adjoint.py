@@ -92,6 +92,32 @@ def test_every_gradient_of_one_object(variant, n_steps):
     adj.close()
 
 
+@pytest.mark.parametrize('variant', [1, 3])
+def test_a_map_and_a_probe_beside_the_gradient(variant):
+    """A field map and a probe change no gradient, and the backward pass leaves the map's sums."""
+    eps = _eps_box()
+    got = []
+    for monitors in (False, True):
+        sim, mon = _product(eps)
+        if monitors:
+            field_map = sim.add_dft_monitor(0.2e-6, 0.1e-6, 1.9e-6, 1.5e-6, wavelengths=[1.0e-6], downsample=2)
+            sim.add_field_probe(1.0e-6, 0.8e-6)
+            sim.em.finalize()
+        sim.em.engine.configure(variant=variant)
+        adj = FluxAdjoint2D(sim, mon, 0, BOX, N_STEPS, checkpoint_every=64)
+        J = adj.forward(eps)
+        if monitors:
+            before = field_map._maps().copy()
+        g = adj.backward()
+        got.append((J, g))
+        if monitors:
+            np.testing.assert_array_equal(field_map._maps(), before)
+            assert np.abs(before).max() > 0
+        adj.close()
+    assert got[0][0] == got[1][0]
+    np.testing.assert_array_equal(got[0][1], got[1][1])
+
+
 def test_torch_autograd_function():
     import torch
     eps = _eps_box()
