@@ -3245,6 +3245,8 @@ extern "C" int os_fdtd2d_adjoint_segment(OsAdjoint2D *a, int32_t slot, int64_t s
     OsFdtd2D *h = a->h;
     OS_CHECK(n_steps >= 1 && n_steps <= a->seg_steps, OS_ERR_INVALID,
              "os_fdtd2d_adjoint_segment: %d steps, the segment holds at most %d", n_steps, a->seg_steps);
+    OS_CHECK(h->tfsf.empty() && h->poles.empty(), OS_ERR_STATE,   // added since os_fdtd2d_adjoint_create
+             "os_fdtd2d_adjoint_segment: the adjoint does not transpose a TFSF box or a dispersive pole");
     OS_CHECK(h->lines.empty() || line_values, OS_ERR_INVALID, "os_fdtd2d_adjoint_segment: line_values is required");
     OS_CHECK(monitor_id >= 0 && monitor_id < (int32_t)h->fluxes.size(), OS_ERR_INVALID,
              "os_fdtd2d_adjoint_segment: no monitor %d", monitor_id);

@@ -118,6 +118,24 @@ def test_a_map_and_a_probe_beside_the_gradient(variant):
     np.testing.assert_array_equal(got[0][1], got[1][1])
 
 
+@pytest.mark.parametrize('feature', ['tfsf', 'pole'])
+def test_a_box_or_a_pole_added_later_is_refused(feature):
+    """What the adjoint does not transpose is refused at the backward pass too, not only when it is created."""
+    eps = _eps_box()
+    sim, mon = _product(eps)
+    adj = FluxAdjoint2D(sim, mon, 0, BOX, 100, checkpoint_every=50)
+    if feature == 'tfsf':
+        sim.add_tfsf(0.4e-6, 0.4e-6, 1.6e-6, 1.2e-6, wavelength=1.0e-6)
+    else:
+        mask = np.zeros((sim.grid.nx, sim.grid.ny), bool)
+        mask[20:24, 30:34] = True
+        sim.add_dispersive(ob.DrudePole(6e14, 2e13), mask)
+    adj.forward(eps)
+    with pytest.raises(RuntimeError, match='does not transpose'):
+        adj.backward()
+    adj.close()
+
+
 def test_torch_autograd_function():
     import torch
     eps = _eps_box()
