@@ -134,14 +134,14 @@ struct OsFdtd2D {
     float dt_hz = 0.0f, eps0_hz = 0.0f;   // dt and eps0 of the lossless form
     int32_t hz_rows = 0;                  // rows per CTA of the fused step kernel (0: chosen per grid)
     int sm_count = 148;                   // multiprocessors of the device (launch sizing)
-    // resident form (fdtd2d_resident_kernel.cuh): the strips' first rows, the boundary rows in flight and their number, the
-    // flux lines' samples of a chunk
+    // resident form (fdtd2d_resident_kernel.cuh): the strips' first rows, the boundary rows in flight and their number (and
+    // behind them the count of blocks that loaded their state), the flux lines' samples of a chunk
     std::vector<int32_t> res_rows;        // host copy of the strips' first rows (empty: not planned)
     os::DeviceArray<int32_t> res_row_start;
     os::DeviceArray<uint64_t> res_mail;
     os::DeviceArray<float> res_stage;
     int32_t res_smem_limit = 0;           // shared memory a block may have
-    uint32_t res_epoch = 1;
+    uint32_t res_epoch = 1, res_arrivals = 0;
 };
 
 namespace os {
@@ -1934,19 +1934,21 @@ static int resident_applies(OsFdtd2D *h, Res2DJob &job, int *shape, size_t *smem
     if (*smem > (size_t)h->res_smem_limit) return OS_OK;
     if (!h->res_row_start.ptr) OS_TRY(upload(h->res_row_start, h->res_rows.data(), h->res_rows.size(), h->stream));
     if (!h->res_mail.ptr) {
-        OS_TRY(h->res_mail.alloc(res2d_mail_words(h->polarization, g.ny, (int)h->res_rows.size() - 1)));
+        OS_TRY(h->res_mail.alloc(res2d_mail_words(h->polarization, g.ny, (int)h->res_rows.size() - 1) + 1));
         OS_CUDA(cudaMemsetAsync(h->res_mail.ptr, 0, h->res_mail.bytes(), h->stream));
         h->res_epoch = 1;
+        h->res_arrivals = 0;
     }
     job.row_start = h->res_row_start.ptr;
     job.mail = h->res_mail.ptr;
+    job.arrived = reinterpret_cast<uint32_t *>(h->res_mail.ptr + h->res_mail.count - 1);
     *yes = true;
     return OS_OK;
 }
 
 // Resident launches of one device are ordered one after another, whatever their streams: each needs the whole chip,
 // and its blocks wait for one another.
-static int launch_resident(OsFdtd2D *h, const Res2DJob &job, int shape, size_t smem) {
+static int launch_resident(OsFdtd2D *h, Res2DJob &job, int shape, size_t smem) {
     static std::mutex mu;
     static cudaEvent_t last[OS_FDTD_MAX_DEVICES] = {};
     OS_CHECK(h->device >= 0 && h->device < OS_FDTD_MAX_DEVICES, OS_ERR_INVALID, "device %d is outside [0, %d)",
@@ -1955,7 +1957,11 @@ static int launch_resident(OsFdtd2D *h, const Res2DJob &job, int shape, size_t s
     cudaEvent_t &ev = last[h->device];
     if (ev) OS_CUDA(cudaStreamWaitEvent(h->stream, ev, 0));
     else OS_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    job.epoch = h->res_epoch;
+    job.arrivals = h->res_arrivals + (uint32_t)job.n_cta;
     OS_CUDA(res2d_launch(shape, job, smem, h->stream));
+    h->res_epoch += (uint32_t)job.n_steps + 1u;
+    h->res_arrivals = job.arrivals;
     OS_CUDA(cudaEventRecord(ev, h->stream));
     h->launches += 1;
     return OS_OK;
@@ -1996,11 +2002,9 @@ static int advance_resident(OsFdtd2D *h, Res2DJob job, int shape, size_t smem, i
         job.n_steps = n;
         job.n0 = h->n_step;
         job.q_first = q_lo;
-        job.epoch = h->res_epoch;
         job.line_values = values + k;
         for (int b = 0; b < job.n_tfsf; ++b) job.tfsf[b].values = values + (h->lines.size() + b) * (size_t)n_steps + k;
         OS_TRY(launch_resident(h, job, shape, smem));
-        h->res_epoch += (uint32_t)n + 1u;
         size_t at = 0;
         for (int f = 0; f < job.n_mons; ++f) {
             FluxLine2D &line = *h->fluxes[f];
@@ -3324,9 +3328,7 @@ extern "C" int os_fdtd2d_adjoint_segment(OsAdjoint2D *a, int32_t slot, int64_t s
         job.rec_i0 = a->bi0, job.rec_i1 = a->bi1, job.rec_j0 = a->bj0, job.rec_j1 = a->bj1;
         job.line_values = a->values.ptr;
         job.values_stride = job.n_steps = n_steps;
-        job.epoch = h->res_epoch;
         OS_TRY(launch_resident(h, job, shape, smem));
-        h->res_epoch += (uint32_t)n_steps + 1u;
     } else if (n_steps == a->seg_steps) {
         const int c = h->cur;
         const Ez2DParams now = make_params(h);

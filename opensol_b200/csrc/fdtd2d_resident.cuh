@@ -63,8 +63,9 @@ struct __align__(16) Res2DJob {
     float *psi_e[4], *psi_h[4];
     const int32_t *row_start;             // n_cta + 1 first rows of the blocks' strips
     uint64_t *mail;                       // boundary rows of the strips (res2d_mail_words)
+    uint32_t *arrived;                    // blocks that ever finished loading their state, this launch's ending at `arrivals`
     uint32_t epoch;                       // number of this chunk's first boundary rows
-    int32_t pad0;
+    uint32_t arrivals;
     int64_t n_steps, n0, m;               // steps of this chunk, steps before it, DFT sample interval
     int64_t q_first;                      // first sample of the chunk (staging slot 0)
     int64_t q_table;                      // first sample of the phase tables

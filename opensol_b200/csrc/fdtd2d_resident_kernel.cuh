@@ -109,6 +109,21 @@ static __device__ __noinline__ bool res_give_up(uint64_t t0, int *err, int *dead
     return true;
 }
 
+// This block has loaded its state, and: have all.
+__device__ __forceinline__ void res_arrive(uint32_t *arrived) {
+    __threadfence();
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(arrived) : "memory");
+}
+static __device__ __noinline__ void res_wait_all(const uint32_t *arrived, uint32_t arrivals, int *err, int *dead) {
+    const uint64_t t0 = tb_globaltimer();
+    for (int tries = 0;; ++tries) {
+        uint32_t n;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(n) : "l"(arrived) : "memory");
+        if ((int32_t)(n - arrivals) >= 0) return;
+        if ((tries & 63) == 63 && res_give_up(t0, err, dead)) return;
+    }
+}
+
 __device__ __forceinline__ float res_wrap_hi(float w) { return w * 1.0f + w * 0.0f; }
 __device__ __forceinline__ float res_wrap_lo(float w) { return w * 1.0f - w * 0.0f; }
 
@@ -1065,7 +1080,6 @@ __global__ void __launch_bounds__(NT, 1) res2d_kernel(const __grid_constant__ Re
     __syncthreads();
 
     ResStrip<HZ, GEN, C, RT> s(p);
-    constexpr int H = C / 2;
     const int c = blockIdx.x, last_cta = p.n_cta - 1;
     s.i0 = p.row_start[c];
     s.R = p.row_start[c + 1] - s.i0;
@@ -1258,6 +1272,7 @@ __global__ void __launch_bounds__(NT, 1) res2d_kernel(const __grid_constant__ Re
     }
     if (HZ) s.publish_hi(s.a);
     else s.publish_lo(s.f);
+    if (tid == 0) res_arrive(p.arrived);   // every thread's loads came before the barrier above
     if (p.stall_probe_ns && c == 0) {
         // test hook: this block sends nothing for the given time, then gives up as a real wait does
         const uint64_t t0 = tb_globaltimer();
@@ -1266,19 +1281,13 @@ __global__ void __launch_bounds__(NT, 1) res2d_kernel(const __grid_constant__ Re
         if (tid == 0) atomicExch(p.err, 1);
         return;
     }
-    // Every value another strip's owner will overwrite (the recomputed row and its psi) has been read: the first mail
-    // says so, and no owner starts its first step before that mail.
     uint32_t epoch = p.epoch;
     s.mail(epoch);
-    {
-        float2 unused[2][H];
-        float none;
-        const uint64_t *const at_q[2] = {s.has_up ? s.from_up + s.slot(epoch) + (HZ ? 2 : 1) * s.mail_p : nullptr,
-                                         s.has_dn ? s.from_dn + s.slot(epoch) : nullptr};
-        s.receive(unused, at_q, none, nullptr, epoch);
-    }
-    __syncthreads();
-    if (dead_flag) return;
+    // No block steps before all have loaded: what one reads here another overwrites later (the recomputed row and its psi
+    // by their owner; the plane-wave boxes' lines, which every block reads, by block 0 at its end, and a mail travels one
+    // strip a step, so a short launch's mails order block 0 behind its near strips only).
+    if (tid == 0) res_wait_all(p.arrived, p.arrivals, p.err, &dead_flag);
+    if (__syncthreads_or(*(volatile int *)&dead_flag)) return;
 
     // ---- the steps
     const bool maps = GEN && HZ && p.n_maps;

@@ -116,6 +116,14 @@ def test_resident_among_the_other_forms(pol):
     _compare(dict(pol=pol, nx=200, ny=164, boundaries='pml', npml=10, seed=7, maps=(3,), probes=2), (20, 31, 25), 1)
 
 
+@pytest.mark.parametrize('pol', ['ez', 'hz'])
+@pytest.mark.parametrize('chunks', [(1,) * 60, (2,) * 30, (1, 2, 3, 30, 1)])
+def test_plane_wave_in_short_launches(pol, chunks):
+    """A plane wave's line is read by every strip and written by one: launches of fewer steps than there are strips, on
+    148 of them, the box reaching from the first strips to the last."""
+    _compare(dict(pol=pol, nx=320, ny=60, boundaries='pml', npml=6, tfsf=2, lines=(), seed=21), chunks)
+
+
 def test_resident_chunk_past_the_staged_samples():
     """A chunk with more DFT samples than one launch stages (every step sampled) runs in several launches."""
     got = []
