@@ -3430,6 +3430,5 @@ extern "C" int os_fdtd2d_adjoint_gradient(OsAdjoint2D *a, double *out) {
     OS_TRY(bind_device(a->h));
     OS_CUDA(cudaMemcpyAsync(out, a->grad.ptr, a->grad.bytes(), cudaMemcpyDeviceToHost, a->adj_stream));
     OS_CUDA(cudaStreamSynchronize(a->adj_stream));
-    OS_CUDA(cudaStreamSynchronize(a->h->stream));
-    return OS_OK;
+    return sync_and_check(a->h);   // a recomputation whose bounded wait ran out has recorded no valid fields
 }

@@ -136,6 +136,24 @@ def test_a_box_or_a_pole_added_later_is_refused(feature):
     adj.close()
 
 
+def test_a_recomputation_that_gave_up_is_reported():
+    """A backward pass whose recomputation left on its bounded wait (the test hook: 1 ms) raises instead of returning a
+    gradient; the next pass is clean."""
+    eps = _eps_box()
+    sim, mon = _product(eps)
+    adj = FluxAdjoint2D(sim, mon, 0, BOX, N_STEPS, checkpoint_every=64)
+    J = adj.forward(eps)
+    g = adj.backward()
+    assert adj.forward(eps) == J
+    sim.em.engine.set_stall_probe(1_000_000)
+    with pytest.raises(RuntimeError, match='bounded wait'):
+        adj.backward()
+    sim.em.engine.set_stall_probe(0)
+    assert adj.forward(eps) == J
+    np.testing.assert_array_equal(adj.backward(), g)
+    adj.close()
+
+
 def test_torch_autograd_function():
     import torch
     eps = _eps_box()
