@@ -121,15 +121,31 @@ void *pool_take(int device, size_t cls) {
 //
 // A read into ordinary memory goes through the driver's staging buffer and one core, which also takes the page faults
 // of a fresh array: 4.7 GB/s (805 MB of 8192 x 8192 fields in 170 ms).  A large read is cut into chunks that several
-// threads fetch into page-locked slots of their own, two each, and copy out while the next chunk travels.  The slots
-// are allocated once per process, used by one read at a time (another read meanwhile takes the plain copy) and freed
-// by pool_trim.
+// threads fetch into page-locked slots of their own, two each, and copy out while the next chunk travels.  The copies
+// go on a stream of the reader's own, behind the caller's stream by an event recorded in the calling thread: another
+// thread may not use the caller's handle (cudaStreamPerThread names a different stream in each).  The slots and streams
+// are made once per process (and device), used by one read at a time (another read meanwhile takes the plain copy) and
+// freed by pool_trim.
 namespace {
 constexpr size_t kReadChunk = (size_t)2 << 20;
 constexpr int kReadThreads = 8;
 constexpr size_t kReadMin = (size_t)4 << 20;   // below, the threads cost more than they save
 std::mutex g_read_mutex;
 unsigned char *g_read_slots = nullptr;   // kReadThreads x 2 chunks, page-locked
+cudaStream_t g_read_streams[OS_FDTD_MAX_DEVICES] = {};
+cudaEvent_t g_read_ready[OS_FDTD_MAX_DEVICES] = {};
+
+// The device's reader stream, behind the work queued on `stream` so far.
+cudaError_t read_stream(int device, cudaStream_t stream, cudaStream_t *out) {
+    cudaStream_t &s = g_read_streams[device];
+    cudaEvent_t &ready = g_read_ready[device];
+    cudaError_t err = s ? cudaSuccess : cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+    if (err == cudaSuccess && !ready) err = cudaEventCreateWithFlags(&ready, cudaEventDisableTiming);
+    if (err == cudaSuccess) err = cudaEventRecord(ready, stream);
+    if (err == cudaSuccess) err = cudaStreamWaitEvent(s, ready, 0);
+    *out = s;
+    return err;
+}
 
 cudaError_t read_chunks(unsigned char *dst, const unsigned char *src, size_t bytes, int device, cudaStream_t stream,
                         unsigned char *slots, std::atomic<size_t> &next) {
@@ -166,22 +182,28 @@ cudaError_t read_chunks(unsigned char *dst, const unsigned char *src, size_t byt
 
 int read_back(void *dst, const void *src, size_t bytes, cudaStream_t stream) {
     std::unique_lock<std::mutex> lock(g_read_mutex, std::defer_lock);
-    if (bytes >= kReadMin && lock.try_lock()) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    int device = -1;
+    if (bytes >= kReadMin) {   // a capturing stream keeps the plain copy, and its error
+        OS_CUDA(cudaGetDevice(&device));
+        OS_CUDA(cudaStreamIsCapturing(stream, &capture));
+    }
+    if (device >= 0 && device < OS_FDTD_MAX_DEVICES && capture == cudaStreamCaptureStatusNone && lock.try_lock()) {
         if (!g_read_slots &&
             cudaHostAlloc((void **)&g_read_slots, kReadThreads * 2 * kReadChunk, cudaHostAllocPortable) != cudaSuccess) {
             g_read_slots = nullptr;
             cudaGetLastError();
         }
         if (g_read_slots) {
-            int device = 0;
-            OS_CUDA(cudaGetDevice(&device));
+            cudaStream_t reader = nullptr;
+            OS_CUDA(read_stream(device, stream, &reader));
             std::atomic<size_t> next{0};
             cudaError_t err[kReadThreads];
             std::vector<std::thread> threads;
             int started = 0;
             auto work = [&](int k) {
                 err[k] = read_chunks(static_cast<unsigned char *>(dst), static_cast<const unsigned char *>(src), bytes,
-                                     device, stream, g_read_slots + k * 2 * kReadChunk, next);
+                                     device, reader, g_read_slots + k * 2 * kReadChunk, next);
             };
             try {
                 threads.reserve(kReadThreads - 1);
@@ -204,6 +226,14 @@ int pool_trim() {
         std::lock_guard<std::mutex> lock(g_read_mutex);
         if (g_read_slots) cudaFreeHost(g_read_slots);
         g_read_slots = nullptr;
+        for (cudaStream_t &s : g_read_streams) {
+            if (s) cudaStreamDestroy(s);
+            s = nullptr;
+        }
+        for (cudaEvent_t &e : g_read_ready) {
+            if (e) cudaEventDestroy(e);
+            e = nullptr;
+        }
     }
     std::vector<PoolBlock> blocks;
     {

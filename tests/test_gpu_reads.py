@@ -1,0 +1,46 @@
+"""Large reads (4 MB and more, which several threads fetch) hold what the work queued before them leaves, whatever the
+caller's stream, and the same values as reads of an engine on its own stream."""
+import numpy as np
+import pytest
+
+import opensol_b200 as ob
+from opensol_b200 import workloads
+
+pytestmark = pytest.mark.gpu
+PER_THREAD = 2   # cudaStreamPerThread: a handle that names another stream in every thread
+CELLS = 1100     # 4.84 MB a field
+STEPS = 600
+
+
+def _sim():
+    sim = ob.Simulation(**workloads.roofline_2d_sim_args(total_cells=CELLS), verbose=False)
+    workloads.apply(sim, workloads.roofline_2d_ops(total_cells=CELLS, n_cylinders=30, seed=5))
+    sim.em.finalize()
+    return sim
+
+
+def _streams():
+    import torch
+    return [PER_THREAD, torch.cuda.Stream().cuda_stream]
+
+
+def _fields(engine):
+    return [engine.read_field(name) for name in ('ez', 'hx', 'hy')]
+
+
+@pytest.mark.parametrize('variant', [1, 3])
+@pytest.mark.parametrize('which', [0, 1])
+def test_read_on_a_callers_stream(variant, which):
+    got = []
+    for stream in (None, _streams()[which]):
+        sim = _sim()
+        engine = sim.em.engine
+        engine.configure(variant=variant)
+        engine.set_stream(stream)
+        engine.advance(STEPS)
+        got.append(_fields(engine))
+        engine.set_stream(None)
+        engine.close()
+    for a, b in zip(*got):
+        np.testing.assert_array_equal(a, b)
+    assert np.abs(got[0][0]).max() > 0
