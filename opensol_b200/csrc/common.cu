@@ -125,7 +125,7 @@ void *pool_take(int device, size_t cls) {
 // go on a stream of the reader's own, behind the caller's stream by an event recorded in the calling thread: another
 // thread may not use the caller's handle (cudaStreamPerThread names a different stream in each).  The slots and streams
 // are made once per process (and device), used by one read at a time (another read meanwhile takes the plain copy) and
-// freed by pool_trim.
+// freed by pool_trim.  Memory that the driver copies to directly (page-locked, managed) takes one plain copy.
 namespace {
 constexpr size_t kReadChunk = (size_t)2 << 20;
 constexpr int kReadThreads = 8;
@@ -134,6 +134,15 @@ std::mutex g_read_mutex;
 unsigned char *g_read_slots = nullptr;   // kReadThreads x 2 chunks, page-locked
 cudaStream_t g_read_streams[OS_FDTD_MAX_DEVICES] = {};
 cudaEvent_t g_read_ready[OS_FDTD_MAX_DEVICES] = {};
+
+bool pageable(const void *p) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return a.type == cudaMemoryTypeUnregistered;
+}
 
 // The device's reader stream, behind the work queued on `stream` so far.
 cudaError_t read_stream(int device, cudaStream_t stream, cudaStream_t *out) {
@@ -184,7 +193,7 @@ int read_back(void *dst, const void *src, size_t bytes, cudaStream_t stream) {
     std::unique_lock<std::mutex> lock(g_read_mutex, std::defer_lock);
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     int device = -1;
-    if (bytes >= kReadMin) {   // a capturing stream keeps the plain copy, and its error
+    if (bytes >= kReadMin && pageable(dst)) {   // a capturing stream keeps the plain copy, and its error
         OS_CUDA(cudaGetDevice(&device));
         OS_CUDA(cudaStreamIsCapturing(stream, &capture));
     }

@@ -44,3 +44,23 @@ def test_read_on_a_callers_stream(variant, which):
     for a, b in zip(*got):
         np.testing.assert_array_equal(a, b)
     assert np.abs(got[0][0]).max() > 0
+
+
+def test_read_into_page_locked_memory():
+    """A page-locked destination takes one direct copy: the same values."""
+    import ctypes
+    from opensol_b200 import _native
+    sim = _sim()
+    engine = sim.em.engine
+    engine.advance(STEPS)
+    want = _fields(engine)
+    lib, p = _native.load(), ctypes.c_void_p()
+    _native.check(lib.os_fdtd_host_alloc(want[0].nbytes, ctypes.byref(p)))
+    try:
+        out = np.frombuffer((ctypes.c_char * want[0].nbytes).from_address(p.value), np.float32).reshape(want[0].shape)
+        for component, field in enumerate(want):
+            out[...] = np.nan
+            _native.check(lib.os_fdtd2d_read_field(engine.handle, component, _native.fptr(out)))
+            np.testing.assert_array_equal(out, field)
+    finally:
+        _native.check(lib.os_fdtd_host_free(p))
