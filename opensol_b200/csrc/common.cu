@@ -1,6 +1,9 @@
 // Thread-local error message and the library-wide entry points of opensol_fdtd.h.
 #include "common.cuh"
 
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <atomic>
 #include <cmath>
 #include <cstring>
@@ -129,11 +132,26 @@ void *pool_take(int device, size_t cls) {
 namespace {
 constexpr size_t kReadChunk = (size_t)2 << 20;
 constexpr int kReadThreads = 8;
-constexpr size_t kReadMin = (size_t)4 << 20;   // below, the threads cost more than they save
+// Below these the threads cost more than they save: into pages not there yet (a fresh array: the copying core also takes
+// their faults, 2 GB/s) and into pages that are.  Measured, us for one plain copy and for the threads: 4.9 MB fresh 2550
+// and 2430, there 290-460 and 540-600; 7.9 MB 4050 and 2700, 425-670 and 620-760; 15.8 MB 8100 and 3500, 800-1250 and
+// 930-1080; 23.8 MB 12000 and 4100, 1160-1930 and 980-1320; 31.8 MB 16000 and 5000, 1560-2850 and 1180-1600.
+constexpr size_t kReadMin = (size_t)4 << 20, kReadMinResident = (size_t)24 << 20;
 std::mutex g_read_mutex;
 unsigned char *g_read_slots = nullptr;   // kReadThreads x 2 chunks, page-locked
 cudaStream_t g_read_streams[OS_FDTD_MAX_DEVICES] = {};
 cudaEvent_t g_read_ready[OS_FDTD_MAX_DEVICES] = {};
+
+// Whether the pages of [p, p + bytes) are there (a sample of them; unknown counts as no).
+bool resident(const void *p, size_t bytes) {
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), first = (uintptr_t)p;
+    for (int k = 0; k < 16; ++k) {
+        unsigned char in = 0;
+        const uintptr_t at = (first + (bytes - 1) / 15 * k) & ~(page - 1);
+        if (mincore((void *)at, page, &in) != 0 || !(in & 1)) return false;
+    }
+    return true;
+}
 
 bool pageable(const void *p) {
     cudaPointerAttributes a;
@@ -193,7 +211,8 @@ int read_back(void *dst, const void *src, size_t bytes, cudaStream_t stream) {
     std::unique_lock<std::mutex> lock(g_read_mutex, std::defer_lock);
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     int device = -1;
-    if (bytes >= kReadMin && pageable(dst)) {   // a capturing stream keeps the plain copy, and its error
+    if (bytes >= kReadMin && pageable(dst) && (bytes >= kReadMinResident || !resident(dst, bytes))) {
+        // a capturing stream keeps the plain copy, and its error
         OS_CUDA(cudaGetDevice(&device));
         OS_CUDA(cudaStreamIsCapturing(stream, &capture));
     }

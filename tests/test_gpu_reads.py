@@ -46,6 +46,26 @@ def test_read_on_a_callers_stream(variant, which):
     assert np.abs(got[0][0]).max() > 0
 
 
+@pytest.mark.parametrize('cells', [1000, 1030, 1100, 2540])
+def test_read_into_fresh_and_used_memory(cells):
+    """Destinations whose pages are there and whose are not take different ways (from 4 and 24 MB: 1000 and 1030, 2540
+    cells a side lie around them): the same values."""
+    import mmap
+    from opensol_b200 import _native
+    sim = ob.Simulation(**workloads.roofline_2d_sim_args(total_cells=cells), verbose=False)
+    sim.em.finalize()
+    engine = sim.em.engine
+    want = np.random.default_rng(cells).standard_normal((engine.nx, engine.ny)).astype(np.float32)
+    engine.write_field('hx', want)
+    lib = _native.load()
+    for used in (False, True):
+        out = np.frombuffer(mmap.mmap(-1, want.nbytes + 4), np.float32)[1:].reshape(want.shape)
+        if used:
+            out[...] = np.nan
+        _native.check(lib.os_fdtd2d_read_field(engine.handle, 1, _native.fptr(out)))
+        np.testing.assert_array_equal(out, want)
+
+
 def test_read_into_page_locked_memory():
     """A page-locked destination takes one direct copy: the same values."""
     import ctypes
