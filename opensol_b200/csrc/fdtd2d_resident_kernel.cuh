@@ -25,8 +25,9 @@
 //
 // GEN adds what plain lossless runs do not need: ca / da / db words, field maps, poles, plane-wave boxes.
 //
-// Every poll is bounded by %globaltimer (2 s): when it runs out the block sets the engine's error flag and leaves, and
-// its neighbours follow when they see the flag or their own bound.
+// Every poll is bounded by %globaltimer: 2 s for a neighbour's mail, 120 s for all blocks to be placed at the start (other
+// streams' kernels may hold multiprocessors until then).  When it runs out the block sets the engine's error flag and
+// leaves, and the others follow when they see the flag or their own bound.
 #pragma once
 
 #include "fdtd2d_resident.cuh"
@@ -100,10 +101,11 @@ __device__ __forceinline__ uint64_t res_peek(const uint64_t *at) {
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(at) : "memory");
     return w;
 }
+#define RES_START_WAIT_NS 120000000000ull
 // Whether a poll that started at t0 gives up: its time is over, or another thread or block gave up (then *dead is set).
-static __device__ __noinline__ bool res_give_up(uint64_t t0, int *err, int *dead) {
+static __device__ __noinline__ bool res_give_up(uint64_t t0, uint64_t wait_ns, int *err, int *dead) {
     if (*(volatile int *)dead) return true;
-    if (!*(volatile int *)err && tb_globaltimer() - t0 <= TB_WAIT_NS) return false;
+    if (!*(volatile int *)err && tb_globaltimer() - t0 <= wait_ns) return false;
     atomicExch(err, 1);
     *(volatile int *)dead = 1;
     return true;
@@ -120,7 +122,7 @@ static __device__ __noinline__ void res_wait_all(const uint32_t *arrived, uint32
         uint32_t n;
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(n) : "l"(arrived) : "memory");
         if ((int32_t)(n - arrivals) >= 0) return;
-        if ((tries & 63) == 63 && res_give_up(t0, err, dead)) return;
+        if ((tries & 63) == 63 && res_give_up(t0, RES_START_WAIT_NS, err, dead)) return;
     }
 }
 
@@ -410,7 +412,7 @@ struct ResStrip {
             extra = __uint_as_float((uint32_t)x);
             if (here) return;
             if (tries == 0) t0 = tb_globaltimer();
-            if ((tries & 63) == 63 && res_give_up(t0, p.err, dead)) return;
+            if ((tries & 63) == 63 && res_give_up(t0, TB_WAIT_NS, p.err, dead)) return;
         }
     }
     __device__ __forceinline__ void send(uint64_t *at, const float2 (&v)[H], uint32_t epoch) {
