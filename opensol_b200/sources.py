@@ -87,11 +87,37 @@ class RickerWavelet:
         return 4.2 * self.f_peak
 
 
+def plain_waveform(temporal):
+    """Whether temporal(float(t)) is a Python float of every t: one of the classes above with plain numbers for parameters
+    (a Gaussian's tau no smaller than its square can be divided by)."""
+    if type(temporal) is GaussianPulse:
+        parameters = (temporal.f0, temporal.t0, temporal.tau if temporal.tau > 1e-100 else None)
+    elif type(temporal) is ContinuousWave:
+        parameters = (temporal.f0, temporal.tau_ramp)
+    elif type(temporal) is RickerWavelet:
+        parameters = (temporal.f_peak, temporal.t0)
+    else:
+        return False
+    return all(isinstance(v, (float, int)) for v in parameters)
+
+
 def temporal_values(temporal, times):
     """float64 temporal(float(t)) per time."""
-    if type(temporal) is GaussianPulse:
+    if type(temporal) is GaussianPulse and plain_waveform(temporal):
         return temporal.at(times)
     return np.array([temporal(float(t)) for t in times], dtype=np.float64)
+
+
+def scaled_values(scale, temporal, times):
+    """float32 scale * temporal(float(t)) per time; as arrays where a product of one value with the scale is that of the
+    arrays (a numpy float32 times a Python float: the value is rounded to float32, then the product)."""
+    if plain_waveform(temporal):
+        values = temporal_values(temporal, times)
+        if isinstance(scale, DTYPE):
+            return scale * values.astype(DTYPE)
+        if type(scale) is float:
+            return (scale * values).astype(DTYPE)
+    return np.array([DTYPE(scale * temporal(float(t))) for t in times], dtype=DTYPE)
 
 
 def make_temporal(waveform, frequency, bandwidth):
@@ -141,8 +167,7 @@ class LineSource:
 
     def values(self, t_half_list):
         """float32 amplitude * temporal(t) per time (the per-step value of LineSource.inject)."""
-        # a numpy float32 times a Python float: the value is rounded to float32, then the product
-        return self.amplitude * temporal_values(self.temporal, t_half_list).astype(DTYPE)
+        return scaled_values(self.amplitude, self.temporal, t_half_list)
 
 
 def sheet_admittance(line_eps, mu_r, sigma_m, omega, normal_spacing, dt):
@@ -297,7 +322,7 @@ class TFSFSource:
 
     def values(self, t_half):
         """float32 soft-source value of each step: FP32(source_scale * temporal(t + dt/2))."""
-        return (self.source_scale * temporal_values(self.temporal, t_half)).astype(DTYPE)
+        return scaled_values(self.source_scale, self.temporal, t_half)
 
 
 def _aux_line_terms(width, dt, half_omega_dt, index=1.0):

@@ -43,3 +43,31 @@ def test_phase_table_equals_one_sample_at_a_time(nf):
         np.testing.assert_array_equal(table[q, :, 0], (np.cos(phase) * (27 * 4.67e-17)).astype(np.float32))
         np.testing.assert_array_equal(table[q, :, 1], (np.sin(phase) * (27 * 4.67e-17)).astype(np.float32))
     assert math.isfinite(float(table.sum())) and dft_phase_table(omega, [], 1.0).shape == (0, nf, 2)
+
+
+class _Numpy:
+    """A waveform whose values are numpy float64 (its product with a numpy float32 is taken in float64)."""
+
+    def __call__(self, t):
+        return np.sin(np.float64(3e14) * t) * np.float64(0.3)
+
+
+@pytest.mark.parametrize('n', [0, 1, 2, 15, 16, 17, 300])
+@pytest.mark.parametrize('temporal, amplitude', [
+    (_Numpy(), None), (GaussianPulse(2e14, 0.5), 0.7), (GaussianPulse(2e14, 0.5), np.float64(0.7)),
+    (GaussianPulse(np.float32(2e14), 0.5), None), (ContinuousWave(np.float32(3e14)), None), (RickerWavelet(2e14), 2)])
+def test_any_waveform_amplitude_and_length(temporal, amplitude, n):
+    """Lengths around the line between the two ways, waveforms of the caller's own, amplitudes set later."""
+    source = LineSource('y', 3, temporal, amplitude=0.7)
+    if amplitude is not None:
+        source.amplitude = amplitude
+    half, full, end = step_clock(2e-15, 4.67e-17, n)
+    x = 2e-15
+    for k in range(n):
+        assert half[k] == x + 0.5 * 4.67e-17
+        x = x + 4.67e-17
+        assert full[k] == x
+    assert end == x and half.shape == full.shape == (n,)
+    got = source.values(half)
+    assert got.dtype == DTYPE and got.shape == (n,)
+    assert got.tolist() == [float(DTYPE(source.amplitude * temporal(float(t)))) for t in half]
