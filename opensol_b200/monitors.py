@@ -47,6 +47,8 @@ def dft_sample_interval(dt, sources, monitor_frequencies, harmonic_order=1) -> i
 def dft_phase_table(omega, times, dt_m):
     """(n_samples, nf, 2) float32 table of complex64 exp(-j omega t) * dt_m per sample time (monitors.py:22-24)."""
     table = np.empty((len(times), omega.size, 2), dtype=np.float32)
+    if len(times) == 0:
+        return table
     phase = -omega[None, :] * np.asarray(times, dtype=np.float64).reshape(-1, 1)
     table[:, :, 0] = np.cos(phase) * float(dt_m)
     table[:, :, 1] = np.sin(phase) * float(dt_m)
@@ -56,6 +58,13 @@ def dft_phase_table(omega, times, dt_m):
 def step_clock(t, dt, n_steps):
     """(t + dt / 2, t + dt) of each of n_steps steps and the clock after them, t accumulated step by step in float64
     (fdtd_ez_2d.py:76-79)."""
+    if n_steps < 16:   # a chunk of a few steps: quicker one by one
+        t_half, t_full = np.empty(n_steps), np.empty(n_steps)
+        for k in range(n_steps):
+            t_half[k] = t + 0.5 * dt
+            t = t + dt
+            t_full[k] = t
+        return t_half, t_full, t
     clock = np.full(n_steps + 1, dt, dtype=np.float64)
     clock[0] = t
     np.add.accumulate(clock, out=clock)

@@ -71,3 +71,20 @@ def test_any_waveform_amplitude_and_length(temporal, amplitude, n):
     got = source.values(half)
     assert got.dtype == DTYPE and got.shape == (n,)
     assert got.tolist() == [float(DTYPE(source.amplitude * temporal(float(t)))) for t in half]
+
+
+def test_short_chunks_take_no_array_detour():
+    """A chunk of one step is as cheap as the loop it restates: no phase arithmetic without samples, no native call."""
+    def refuse(*_):
+        raise AssertionError('a chunk of one step went through the arrays')
+    pulse = GaussianPulse(2e14, 0.5)
+    pulse.at = refuse
+    LineSource('y', 3, pulse).values(step_clock(0.0, 4.67e-17, 1)[0])
+
+    class Omega:
+        size = 4
+
+        def __neg__(self):
+            refuse()
+        __getitem__ = __mul__ = __rmul__ = refuse
+    assert dft_phase_table(Omega(), [], 1.0).shape == (0, 4, 2)
