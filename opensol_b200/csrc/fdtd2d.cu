@@ -1892,11 +1892,26 @@ static Res2DJob resident_job(const OsFdtd2D *h) {
     return p;
 }
 
-// Whether the handle's chunks run in the resident form now (job, shape and smem filled), planning its strips on the
-// first call.  It takes every feature of the per-step kernels within the parameter block's limits, on any grid whose
+// Steps a chunk of strips of `rows` rows must have for the resident form: a launch reads and writes all of its strips'
+// state, about 20 us and 3 us a row (an H_z launch at best 28 us, against 25 of one step of the blocked kernels).  Measured,
+// us per step here and in the blocked kernels: E_z 4 rows 1 step 31, 31; 8 rows 1 step 44, 33, 3 steps 18.4, 15.9, 5 steps
+// 13.2, 15.0; 13 rows 5 steps 17.2, 14.5, 10 steps 12.3, 14.1; 20 rows 10 steps 15.2, 13.0, 20 steps 12.3, 12.4; 24 rows 20
+// steps 14.4, 13.6, 40 steps 12.5, 13.6; H_z 4 rows 1 step 31.7, 25.4, 2 steps 17.2, 18.7; 8 rows 3 steps 20.3, 20.9.  The
+// general kernels gain less a step (maps, 13 rows: 10 steps 14.2, 14.0).  Probes and maps are launches of their own in the
+// blocked kernels (6 rows, 2 steps, probe: 20.2, 19.8; H_z 21.2, 22.8).  Against launches per half step (poles, plane-wave
+// boxes): 5 rows 1 step 42, 42; H_z 3 rows 1 step 36, 40.
+static int64_t resident_min_steps(const OsFdtd2D *h, int rows, bool blocked, bool general) {
+    if (!blocked || (rows <= 6 && (h->probes.n || !h->maps.empty()))) return (rows + 3) / 4;
+    if (rows <= 4) return h->polarization == 1 ? 2 : 1;
+    if (rows > 17) return 2 * rows - 20;
+    return general && rows > 8 ? rows + 1 : (rows + 1) / 2;
+}
+
+// Whether a chunk of n_steps of the handle runs in the resident form now (job, shape and smem filled), planning its strips
+// on the first call.  It takes every feature of the per-step kernels within the parameter block's limits, on any grid whose
 // strips fit a kernel shape (registers: 1.3 to 2 M cells) and a multiprocessor's shared memory; stream capture keeps the
 // launch-per-step forms, whose work a captured graph may replay beside other kernels.
-static int resident_applies(OsFdtd2D *h, Res2DJob &job, int *shape, size_t *smem, bool *yes) {
+static int resident_applies(OsFdtd2D *h, int64_t n_steps, Res2DJob &job, int *shape, size_t *smem, bool *yes) {
     *yes = false;
     const OsGrid2D &g = h->grid;
     if (!h->automatic || h->profiling || g.nx < 2 || g.ny < 2) return OS_OK;
@@ -1922,6 +1937,7 @@ static int resident_applies(OsFdtd2D *h, Res2DJob &job, int *shape, size_t *smem
     *shape = res2d_shape(g.ny, max_rows, blocked);
     if (*shape < 0) return OS_OK;
     job = resident_job(h);
+    if (n_steps < resident_min_steps(h, max_rows, blocked, res2d_general(job))) return OS_OK;
     const bool lo = g.cpml_sides & 1, hi = g.cpml_sides & 2;
     auto rows_in = [](int a, int b, int c, int d) { return std::max(0, std::min(b, d) - std::max(a, c)); };
     *smem = 0;
@@ -2052,7 +2068,7 @@ static int run_chunk(OsFdtd2D *h, int64_t n_steps, int64_t first_sample, int64_t
     Res2DJob job{};
     int shape = -1;
     size_t smem = 0;
-    if (may_allocate) OS_TRY(resident_applies(h, job, &shape, &smem, &resident));
+    if (may_allocate) OS_TRY(resident_applies(h, n_steps, job, &shape, &smem, &resident));
     // a TFSF box or a pole acts between the H and E updates of every step: the per-half-step kernels run them
     const int rc = resident ? advance_resident(h, job, shape, smem, n_steps, first_sample, n_samples, values,
                                                phase_table)
@@ -3012,7 +3028,7 @@ extern "C" int os_fdtd2d_batch_advance(OsFdtd2DBatch *b, OsFdtd2D *const *handle
     std::vector<Resident> runs((size_t)n_jobs);
     bool all = true;
     for (int32_t q = 0; q < n_jobs && all; ++q)
-        OS_TRY(resident_applies(handles[q], runs[q].job, &runs[q].shape, &runs[q].smem, &all));
+        OS_TRY(resident_applies(handles[q], n_steps, runs[q].job, &runs[q].shape, &runs[q].smem, &all));
     if (!all) {
         OS_TRY(batch_advance_blocked(b, handles, n_jobs, n_steps, line_values, first_samples, n_samples, phases));
     } else {
@@ -3318,7 +3334,7 @@ extern "C" int os_fdtd2d_adjoint_segment(OsAdjoint2D *a, int32_t slot, int64_t s
     int shape = -1;
     size_t smem = 0;
     bool resident = false;
-    OS_TRY(resident_applies(h, job, &shape, &smem, &resident));
+    OS_TRY(resident_applies(h, n_steps, job, &shape, &smem, &resident));
     if (resident) {   // the whole segment in one launch, the box recorded by the launch (the state only: no samples, for
                       // which it has no tables: flux lines, probes and field maps keep the forward run's)
         ez2d_record_box_kernel<<<(unsigned)((box + 255) / 256), 256, 0, s>>>(h->ez[h->cur].ptr, h->grid.ny, a->bi0,

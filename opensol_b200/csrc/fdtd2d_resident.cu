@@ -24,9 +24,13 @@ size_t res2d_mail_words(int hz, int ny, int n_cta) {
     return (size_t)n_cta * 2 * res_mail_rows(hz) * (size_t)res_pitch(ny);
 }
 
-cudaError_t res2d_launch(int shape, const Res2DJob &job, size_t smem, cudaStream_t stream) {
+bool res2d_general(const Res2DJob &job) {
     // a uniform da other than 1 has no array, but scales H all the same: the general kernels multiply by it
-    const bool gen = job.ca || job.da || job.da_u != 1.0f || job.n_maps || job.n_poles || job.n_tfsf;
+    return job.ca || job.da || job.da_u != 1.0f || job.n_maps || job.n_poles || job.n_tfsf;
+}
+
+cudaError_t res2d_launch(int shape, const Res2DJob &job, size_t smem, cudaStream_t stream) {
+    const bool gen = res2d_general(job);
     if (job.hz) return gen ? res2d_launch_hz_gen(shape, job, smem, stream) : res2d_launch_hz_plain(shape, job, smem, stream);
     return gen ? res2d_launch_ez_gen(shape, job, smem, stream) : res2d_launch_ez_plain(shape, job, smem, stream);
 }

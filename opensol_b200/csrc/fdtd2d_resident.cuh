@@ -94,5 +94,7 @@ int res2d_shape(int ny, int max_rows, bool blocked_takes_it);
 size_t res2d_smem_bytes(const Res2DJob &job, int i0, int i1, int layer_e, int layer_h, int shape);
 // 64-bit words of a simulation's mail.
 size_t res2d_mail_words(int hz, int ny, int n_cta);
+// Whether the job runs in the kernels with conductivity, magnetic cells, maps, poles and plane-wave boxes.
+bool res2d_general(const Res2DJob &job);
 // Launches one simulation (n_cta blocks of `smem` bytes, the largest strip's).
 cudaError_t res2d_launch(int shape, const Res2DJob &job, size_t smem, cudaStream_t stream);

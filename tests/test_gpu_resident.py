@@ -68,9 +68,9 @@ def _outputs(sim, out):
     return got
 
 
-def _compare(args, chunks, switch=None):
+def _compare(args, chunks, switch=None, resident=None):
     """chunks of steps in the resident form and in variant 0 from the same seeded fields; `switch`: after that chunk the
-    resident engine continues with the blocked kernels and then goes back."""
+    resident engine continues with the blocked kernels and then goes back; `resident`: which chunks run resident (all)."""
     sim, out = _sim(**args)
     ref, ref_out = _sim(**args)
     ref.em.engine.configure(variant=0)
@@ -79,7 +79,9 @@ def _compare(args, chunks, switch=None):
             sim.em.engine.configure(variant=1 if k == switch else 3)
         sim.em.engine.advance(n)
         launches = sim.em.engine.launch_count()
-        if switch is None or k != switch:
+        if resident is not None and not resident[k]:
+            assert launches != 1   # the flux lines' folds aside, a resident chunk is one launch
+        elif switch is None or k != switch:
             assert launches <= 1 + 3   # one resident launch, one fold per flux line
         ref.em.engine.advance(n)
     for a, b in zip(_outputs(sim, out), _outputs(ref, ref_out)):
@@ -122,6 +124,22 @@ def test_plane_wave_in_short_launches(pol, chunks):
     """A plane wave's line is read by every strip and written by one: launches of fewer steps than there are strips, on
     148 of them, the box reaching from the first strips to the last."""
     _compare(dict(pol=pol, nx=320, ny=60, boundaries='pml', npml=6, tfsf=2, lines=(), seed=21), chunks)
+
+
+# rows a strip, steps of the shortest resident chunk (E_z, H_z), features
+RULE = [(4, 1, 2, {}), (5, 3, 3, {}), (8, 4, 4, {}), (13, 7, 7, {}), (17, 9, 9, {}), (20, 20, 20, {}),
+        (6, 2, 2, dict(probes=1)), (7, 4, 4, dict(probes=1)), (6, 2, 2, dict(maps=(5,))), (8, 4, 4, dict(maps=(5,)))]
+
+
+@pytest.mark.parametrize('pol', ['ez', 'hz'])
+@pytest.mark.parametrize('rows, ez_steps, hz_steps, features', RULE)
+def test_short_chunks_take_the_quicker_form(pol, rows, ez_steps, hz_steps, features):
+    """A chunk runs resident from the length at which its launch pays for reading and writing the strips' state; chunks
+    on both sides of the line continue one run."""
+    least = hz_steps if pol == 'hz' else ez_steps
+    args = dict(pol=pol, nx=148 * rows - 12 - 2 * rows, ny=36, boundaries='pml', npml=6, seed=rows, **features)
+    chunks = [n for n in (least, least - 1, least + 1, max(1, least - 1)) if n]
+    _compare(args, chunks, resident=[n >= least for n in chunks])
 
 
 def test_resident_chunk_past_the_staged_samples():
