@@ -14,6 +14,8 @@ int res2d_shape(int ny, int max_rows, bool blocked_takes_it) {
     return -1;
 }
 
+int res2d_columns(int shape) { return RES_SHAPES[shape].c; }
+
 size_t res2d_smem_bytes(const Res2DJob &job, int i0, int i1, int layer_e, int layer_h, int shape) {
     return sizeof(Res2DJob) + (size_t)(i1 - i0 + 2) * sizeof(ResRow) +
            (size_t)job.n_poles * sizeof(ResPoleRows) +

@@ -90,6 +90,8 @@ static_assert(sizeof(Res2DJob) % 16 == 0, "Res2DJob lies in front of 16-byte vec
 // Kernel shape for strips of max_rows rows of ny columns, -1 when they fit none (or, for a run that the blocked kernels
 // take too, none that is faster than those).
 int res2d_shape(int ny, int max_rows, bool blocked_takes_it);
+// Columns a thread of a shape.
+int res2d_columns(int shape);
 // Shared memory of the block of rows [i0, i1), layer_e / layer_h of them in the E / H kind's x-side CPML.
 size_t res2d_smem_bytes(const Res2DJob &job, int i0, int i1, int layer_e, int layer_h, int shape);
 // 64-bit words of a simulation's mail.

@@ -142,6 +142,20 @@ def test_short_chunks_take_the_quicker_form(pol, rows, ez_steps, hz_steps, featu
     _compare(args, chunks, resident=[n >= least for n in chunks])
 
 
+# polarisation, features, rows a strip up to which the general kernels run them, columns
+TALL = [('hz', dict(lossy=True), 9, 60), ('ez', dict(lossy=True), 17, 60), ('hz', dict(magnetic=True), 9, 60),
+        ('ez', dict(magnetic=True), 9, 60), ('ez', dict(magnetic=True), 17, 260), ('hz', dict(maps=(3,)), 16, 60),
+        ('ez', dict(maps=(3,)), 17, 60), ('ez', dict(poles=(DRUDE,)), 14, 60), ('hz', dict(poles=(DRUDE,)), 12, 60),
+        ('ez', dict(poles=(LORENTZ,)), 12, 820), ('hz', dict(poles=(LORENTZ,)), 8, 1340)]
+
+
+@pytest.mark.parametrize('pol, features, rows, ny', TALL)
+def test_tall_strips_take_the_quicker_form(pol, features, rows, ny):
+    for r in (rows, rows + 1):
+        args = dict(pol=pol, nx=148 * r - 12 - 2 * r, ny=ny - 12, boundaries='pml', npml=6, seed=r, **features)
+        _compare(args, (45, 2 * rows + 2), resident=[r == rows] * 2)
+
+
 def test_resident_chunk_past_the_staged_samples():
     """A chunk with more DFT samples than one launch stages (every step sampled) runs in several launches."""
     got = []
