@@ -1907,21 +1907,25 @@ static int64_t resident_min_steps(const OsFdtd2D *h, int rows, bool blocked, boo
     return general && rows > 8 ? rows + 1 : (rows + 1) / 2;
 }
 
-// Rows a strip up to which the general kernels beat the alternative (they spill more, the taller the strip; the plain ones
-// win at every shape they are used for).  Measured at 100 to 730 columns, us per step here and in the blocked kernels:
-// conductivity H_z 9 rows 9.5-12.4, 12.5-16.6, 11 rows 10.7-15.3, 12.5-16.6, 13 rows 11.9-19.5, 12.5-20.7, 22 rows 19-27,
-// 12.5-16.7; E_z 17 rows 11.2-12.6, 12.6-17.5, 22 rows 13.8-21.7, 12.7-16.5; magnetic cells E_z 100 columns 9 rows 7.8, 8.4, 11
-// rows 9.2, 8.4, 330 and 470 columns 17 rows 12.0 and 14.2, 20.7 and 26.8; H_z 9 rows 9.6-11.9, 13.9-18.2, 12 rows 12.1-18.4,
-// 14.5-18.6; maps H_z 16 rows 14.2-15.4, 14.8-17.6, 18 rows 15.4-16.5, 14.8-18.1; E_z 17 rows 11.4-12.7, 11.9-16.2.  Against
-// launches per half step, with poles: E_z 14 rows 20.5-22.4, 24.7-29.0, 16 rows 25.9, 24.7 (100 columns), four columns a thread
-// 12 rows 33.4-37.3, 39.1, 14 rows 39.9-43.4, 42.2; H_z 12 rows 28-31, 31-40, 14 rows 36, 32, four columns 8 rows 36-46, 44-53,
-// 10 rows 51-59, 47.  Plane-wave boxes alone win at every height (20 rows, 100 columns 26-30, 32).
+// Rows a strip up to which the resident form beats the alternative (the taller the strip, the more its kernels spill).
+// Measured at 60 to 730 columns, us per step here and in the blocked kernels.  Plain, columns a multiple of 4 (the blocked
+// kernels' staged rows): E_z 20 rows 11.8, 11.8, 22 rows 12.6, 11.8; H_z 22 rows 12.5-13.0, 12.6-13.0, 23 rows 13.7, 13.1; other
+// columns win at every height (22 rows 11.7-12.4, 13.6-16.4).  Conductivity H_z 9 rows 9.5-12.4, 12.5-16.6, 11 rows 10.7-15.3,
+// 12.5-16.6, 13 rows 11.9-19.5, 12.5-20.7, above 1024 columns (blocks of 640 threads) 7 rows 14.2-14.7, 12.6; E_z 17 rows
+// 11.2-12.6, 12.6-17.5, 22 rows 13.8-21.7, 12.7-16.5.  Magnetic cells E_z 100 columns 9 rows 7.8, 8.4, 11 rows 9.2, 8.4, 280
+// columns 15 rows 17.6, 16.6, 330 and 470 columns 17 rows 12.0 and 14.2, 20.7 and 26.8; H_z 9 rows 9.6-11.9, 13.9-18.2, 12 rows
+// 12.1-18.4, 14.5-18.6.  Maps H_z 16 rows 14.2-15.4, 14.8-17.6, 18 rows 15.4-16.5, 14.8-18.1; E_z 17 rows 11.4-12.7, 11.9-16.2.
+// Against launches per half step, with poles: E_z 14 rows 20.5-22.4, 24.7-29.0, 16 rows 25.9, 24.7 (100 columns), four columns a
+// thread 12 rows 33.4-37.3, 39.1, 14 rows 39.9-43.4, 42.2; H_z 12 rows 28-31, 31-40, 14 rows 36, 32, four columns 8 rows 36-46,
+// 44-53, 10 rows 51-59, 47; plane-wave boxes alone 20 rows of 100 columns 26-30, 32, 14 rows of 60 columns 27.8, 26.8.
 static int resident_max_rows(const OsFdtd2D *h, const Res2DJob &job, int columns) {
     const bool hz = h->polarization == 1;
+    const int ny = h->grid.ny;
     if (job.n_poles) return columns == 2 ? (hz ? 12 : 14) : (hz ? 8 : 12);
-    if (job.n_tfsf || !res2d_general(job)) return INT32_MAX;
-    if (hz) return job.ca || job.da ? 9 : 16;
-    return job.da && h->grid.ny <= 256 ? 9 : 17;
+    if (job.n_tfsf) return ny < 96 ? 12 : INT32_MAX;
+    if (!res2d_general(job)) return ny % 4 ? INT32_MAX : (hz ? 22 : 20);
+    if (hz) return job.ca || job.da ? (ny > 1024 ? 5 : 9) : 16;
+    return job.da && ny < 300 ? 9 : 17;
 }
 
 // Whether a chunk of n_steps of the handle runs in the resident form now (job, shape and smem filled), planning its strips

@@ -142,9 +142,10 @@ def test_short_chunks_take_the_quicker_form(pol, rows, ez_steps, hz_steps, featu
     _compare(args, chunks, resident=[n >= least for n in chunks])
 
 
-# polarisation, features, rows a strip up to which the general kernels run them, columns
-TALL = [('hz', dict(lossy=True), 9, 60), ('ez', dict(lossy=True), 17, 60), ('hz', dict(magnetic=True), 9, 60),
-        ('ez', dict(magnetic=True), 9, 60), ('ez', dict(magnetic=True), 17, 260), ('hz', dict(maps=(3,)), 16, 60),
+# polarisation, features, rows a strip up to which they run resident, columns
+TALL = [('ez', {}, 20, 64), ('hz', {}, 22, 64), ('hz', dict(lossy=True), 5, 1040), ('ez', dict(tfsf=1, lines=()), 12, 60),
+        ('hz', dict(lossy=True), 9, 60), ('ez', dict(lossy=True), 17, 60), ('hz', dict(magnetic=True), 9, 60),
+        ('ez', dict(magnetic=True), 9, 60), ('ez', dict(magnetic=True), 17, 302), ('hz', dict(maps=(3,)), 16, 60),
         ('ez', dict(maps=(3,)), 17, 60), ('ez', dict(poles=(DRUDE,)), 14, 60), ('hz', dict(poles=(DRUDE,)), 12, 60),
         ('ez', dict(poles=(LORENTZ,)), 12, 820), ('hz', dict(poles=(LORENTZ,)), 8, 1340)]
 
