@@ -1,4 +1,4 @@
-"""The resident form of the 2D step (a whole chunk in one launch, fields in shared memory; what a new engine runs where
+"""The resident form of the 2D step (a whole chunk in one launch, fields in registers; what a new engine runs where
 the grid fits) against the per-half-step kernels (variant 0), which the oracle and open_sol's fixtures pin: fields,
 spectra, maps and probe series bit for bit, on strips of one row and of many, every boundary preset, odd rows, lossy
 and magnetic cells, plane-wave boxes, poles, chunk ends on and off DFT samples, and switches between the forms."""
@@ -95,7 +95,7 @@ CASES = [
     dict(nx=120, ny=75, boundaries='pml', npml=10),
     dict(nx=127, ny=64, boundaries='pml', npml=10, lossy=True, probes=3),            # 147 strips of one row
     dict(nx=129, ny=33, boundaries='pml', npml=10, magnetic=True, probes=2),         # 149 rows: strips of one and two
-    dict(nx=300, ny=1200, boundaries='pml', npml=15, maps=(3,)),                     # several columns a thread
+    dict(nx=300, ny=1200, boundaries='pml', npml=15, maps=(3,)),                     # blocks of 640 threads
     dict(nx=777, ny=129, boundaries='periodic_y', npml=15, maps=(1,), probes=1),
     dict(nx=150, ny=131, boundaries='periodic_x', npml=8, lines=('x', 'y'), maps=(2,)),
     dict(nx=149, ny=90, boundaries='periodic', npml=15, lossy=True, magnetic=True),
@@ -124,6 +124,49 @@ def test_plane_wave_in_short_launches(pol, chunks):
     """A plane wave's line is read by every strip and written by one: launches of fewer steps than there are strips, on
     148 of them, the box reaching from the first strips to the last."""
     _compare(dict(pol=pol, nx=320, ny=60, boundaries='pml', npml=6, tfsf=2, lines=(), seed=21), chunks)
+
+
+# One set of grids per kernel shape (columns a thread, rows a strip, threads) of the launch table; cells a side with the
+# CPML, so that the columns leave 1, 2 and 3 over whole threads.
+SHAPES = {
+    (2, 8, 640): [dict(nx=1100, ny=1131, boundaries='pml'), dict(nx=700, ny=1050, boundaries='periodic_y', lossy=True),
+                  dict(nx=1020, ny=1203, boundaries='periodic_x', maps=(7,), probes=2)],
+    (2, 16, 384): [dict(nx=2300, ny=301, boundaries='pml', probes=3), dict(nx=1330, ny=90, boundaries='periodic', lossy=True),
+                   dict(nx=1900, ny=203, boundaries='periodic_y', maps=(5,)), dict(nx=1500, ny=77, boundaries='pml', tfsf=2,
+                                                                                   lines=())],
+    (2, 24, 256): [dict(nx=2900, ny=121, boundaries='pml'), dict(nx=2700, ny=63, boundaries='periodic_y', probes=1),
+                   dict(nx=2800, ny=130, boundaries='pml', tfsf=1, lines=())],
+    (4, 4, 640): [dict(nx=560, ny=1501, boundaries='pml', tfsf=1, lines=(), poles=('drude', 'lorentz'), probes=2),
+                  dict(nx=300, ny=1402, boundaries='periodic_y', poles=('lorentz',), lossy=True, maps=(6,)),
+                  dict(nx=420, ny=1999, boundaries='periodic_x', poles=('drude', 'drude'), lines=('x', 'y'))],
+    (4, 8, 512): [dict(nx=760, ny=1501, boundaries='pml', tfsf=1, lines=(), poles=('drude', 'lorentz')),
+                  dict(nx=700, ny=1402, boundaries='periodic_y', poles=('lorentz',), magnetic=True),
+                  dict(nx=1000, ny=1299, boundaries='periodic', poles=('drude',), maps=(9,))],
+    (4, 10, 384): [dict(nx=1400, ny=901, boundaries='pml', tfsf=2, lines=(), probes=2),
+                   dict(nx=1450, ny=1002, boundaries='pml', tfsf=1, lines=('y',), maps=(8,)),
+                   dict(nx=1350, ny=1503, boundaries='periodic_y', tfsf=1)],
+    (4, 16, 256): [dict(nx=2200, ny=801, boundaries='pml', tfsf=1, lines=()),
+                   dict(nx=1650, ny=1002, boundaries='periodic_y', tfsf=2, maps=(9,)),
+                   dict(nx=1580, ny=903, boundaries='periodic_x', tfsf=1, lossy=True, lines=('x',))],
+}
+
+
+@pytest.mark.parametrize('pol', ['ez', 'hz'])
+@pytest.mark.parametrize('shape, case', [(shape, k) for shape in SHAPES for k in range(len(SHAPES[shape]))])
+def test_every_kernel_shape(pol, shape, case):
+    args = dict(SHAPES[shape][case], pol=pol, seed=50 + case, npml=7)
+    for axis, n in (('x', 'nx'), ('y', 'ny')):
+        if args['boundaries'] not in ('periodic', f'periodic_{axis}'):
+            args[n] -= 14
+    args['poles'] = tuple({'drude': DRUDE, 'lorentz': LORENTZ}[p] for p in args.get('poles', ()))
+    _compare(args, (24, 20, 25))
+    # the shapes before this one in the table do not fit, so the launch used it
+    tall, wide = -(-SHAPES[shape][case]['nx'] // 148), SHAPES[shape][case]['ny']
+    table = [(2, 4, 640), (2, 8, 512), (2, 8, 640), (4, 4, 640), (2, 16, 384), (4, 8, 512), (2, 24, 256), (4, 10, 384),
+             (4, 16, 256)]
+    fits = [s for s in table if tall <= s[1] and -(-wide // s[0]) <= s[2]
+            and (s[0] == 2 or args['poles'] or args.get('tfsf'))]
+    assert fits[0] == shape
 
 
 # rows a strip, steps of the shortest resident chunk (E_z, H_z), features
@@ -201,6 +244,34 @@ def test_resident_engines_share_the_device():
             alone.em.engine.advance(40)
         for x, y in zip(_outputs(sim, out), _outputs(alone, alone_out)):
             np.testing.assert_array_equal(x, y)
+
+
+@pytest.mark.parametrize('pol', ['ez', 'hz'])
+def test_resident_passes_repeat(pol):
+    """Whole passes from rest on one engine, with other engines' passes queued between: every pass gives the same bits,
+    those of the per-step kernels."""
+    runs = [dict(nx=250, ny=131, boundaries='pml', npml=8, lossy=True, probes=2, maps=(3,)),
+            dict(nx=300, ny=90, boundaries='pml', npml=8, tfsf=1, lines=(), poles=(DRUDE, LORENTZ), maps=(2,)),
+            dict(nx=900, ny=203, boundaries='periodic_y', npml=8, probes=1),
+            dict(nx=700, ny=1300, boundaries='pml', npml=8, poles=(LORENTZ,))]
+    sims = [_sim(pol=pol, seed=30 + k, **args) for k, args in enumerate(runs)]
+    first = [None] * len(runs)
+    for repeat in range(3):
+        for sim, _out in sims:
+            sim.em.engine.reset()
+            for n in (60, 31):
+                sim.em.engine.advance(n)
+        for k, (sim, out) in enumerate(sims):
+            got = [np.array(a) for a in _outputs(sim, out)]
+            if repeat == 0:
+                ref, ref_out = _sim(pol=pol, seed=30 + k, **runs[k])
+                ref.em.engine.configure(variant=0)
+                ref.em.engine.reset()
+                for n in (60, 31):
+                    ref.em.engine.advance(n)
+                first[k] = [np.array(a) for a in _outputs(ref, ref_out)]
+            for a, b in zip(got, first[k]):
+                np.testing.assert_array_equal(a, b)
 
 
 def test_resident_bounded_wait():
