@@ -430,7 +430,7 @@ int os_fdtd3d_set_x_chunk(OsFdtd3D *h, int32_t planes);
  * two-kernel update of that layer, on two field sets and two CPML psi sets swapped every step (twice the field memory,
  * a third less DRAM traffic per step); 2 = form 1 with each x plane of a tile staged in shared memory by tensor copies
  * (rows of a multiple of 8 cells, at least 48; other grids run form 1); 3 (the default) = form 1 with the lean staged
- * kernel (four cells a thread; z rows of a multiple of 4 cells and at least 144, y at least 17, at most 255 z CPML
+ * kernel (four cells a thread; z rows of a multiple of 8 cells and at least 144, y at least 17, at most 255 z CPML
  * rows; other grids run form 0). */
 int os_fdtd3d_set_variant(OsFdtd3D *h, int32_t variant);
 

@@ -7,7 +7,7 @@
 //     em3d_lean_kernel (fdtd3d_lean.cuh) does H and E of every cell but the outermost x and y layers (and the z faces
 //     too on an open z axis) in one pass over tensor-copy-staged planes, four cells a thread; the outer layers run
 //     em3d_h_kernel, then em3d_e_kernel, per face in block shapes of their own; em3d_dipole_kernel adds the dipoles.
-//     Rows of a multiple of 4 cells, at least 144; other grids run variant 0;
+//     Rows of a multiple of 8 cells, at least 144; other grids run variant 0;
 //   variant 0: em3d_h_kernel then em3d_e_kernel over the whole grid, in place on one field set;
 //   variant 1: variant 3's schedule with em3d_fused_kernel, one cell a thread (every cell but the outermost layer of
 //     each axis), the faces by the face kernels;
@@ -210,10 +210,10 @@ static Em3DBox fused_box(const OsFdtd3D *h) {
     return Em3DBox{1, g.nx - 1, 1, g.ny - 1, 1, g.nz - 1};
 }
 
-// variant 3's lean kernel: rows of a multiple of 4 cells (16-byte vectors), boxes no larger than the grid (the id box
-// is 144 cells wide, the tallest 17 rows), z CPML rows that fit one byte.
+// variant 3's lean kernel: rows of a multiple of 8 cells (16-byte vectors; the 16-bit id rows are a multiple of 16 bytes, as
+// a tensor map's stride must be), boxes no larger than the grid (the id box is 144 cells wide, the tallest 17 rows), z CPML rows that fit one byte.
 static bool lean_ok(const OsFdtd3D *h) {
-    return h->grid.nz % 4 == 0 && h->grid.nz >= Em3DLeanLayout<16>::WM && h->grid.ny >= 17 &&
+    return h->grid.nz % 8 == 0 && h->grid.nz >= Em3DLeanLayout<16>::WM && h->grid.ny >= 17 &&
            h->cpml[2].nr <= EM3D_LEAN_MAX_ZROWS;
 }
 

@@ -35,7 +35,7 @@
 // nz - 1 is the cell's own.
 //
 // Every wait is bounded (2 s): a block whose wait runs out sets *err, waits (bounded) for its own copies in flight and
-// returns; ids read from a slot are clamped below n_ids.  Needs nz a multiple of 4 and at least 144, ny at least
+// returns; ids read from a slot are clamped below n_ids.  Needs nz a multiple of 8 and at least 144, ny at least
 // TY + 1 (a tensor map's box may not be larger than the array), at most EM3D_LEAN_MAX_ZROWS z CPML rows and chunks of
 // at most EM3D_LEAN_MAX_PLANES - 1 planes.
 #pragma once

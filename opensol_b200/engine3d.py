@@ -289,7 +289,7 @@ class FDTDEngine3D:
         """Step form (speed and memory only; results are bit-identical): 0 = the two in-place kernels, 1 = the fused
         kernel on two field and psi sets, 2 = the fused kernel with its planes staged in shared memory by tensor
         copies (rows of a multiple of 8 cells; other grids run form 1), 3 = the lean staged fused kernel (the default:
-        four cells a thread, packed arithmetic; z rows of a multiple of 4 cells and at least 144, y at least 17; other
+        four cells a thread, packed arithmetic; z rows of a multiple of 8 cells and at least 144, y at least 17; other
         grids run form 0)."""
         _native.check(_native.load().os_fdtd3d_set_variant(self.handle, int(variant)))
 

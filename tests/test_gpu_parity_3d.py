@@ -73,6 +73,27 @@ def test_chunking_and_reset(spec):
     assert engine.n_step == n
 
 
+@pytest.mark.parametrize('nz', [144, 148, 152, 156, 165])
+def test_rows_of_any_length(nz):
+    """Rows of 144 cells and more in the default form: the lean kernels' 16-bit id rows must be a multiple of 16 bytes, so
+    lengths that leave 4 over 8 run the in-place form, as odd ones do."""
+    runs = []
+    for variant in (None, 0):
+        physics, monitors = build_product(dict(CASES3D[1], name=f'c3_mixed_nz{nz}', window=(16, 20, nz - 10)))
+        engine = physics.engine
+        assert engine.shape[2] == nz
+        if variant is not None:
+            engine.set_variant(variant)
+        physics.run(21)
+        assert engine.interior()[1] == (variant is None and nz % 8 == 0)
+        runs.append((engine.state(), [np.asarray(m.flux()) for m in monitors]))
+    for name in FIELDS:
+        np.testing.assert_array_equal(runs[0][0][name], runs[1][0][name], err_msg=name)
+    for f0, f1 in zip(runs[0][1], runs[1][1]):
+        np.testing.assert_array_equal(f0, f1)
+    assert max(np.abs(runs[0][0][name]).max() for name in FIELDS) > 0
+
+
 def test_field_roundtrip_and_launches():
     spec = CASES3D[0]
     physics, _ = build_product(spec)
