@@ -3091,6 +3091,7 @@ extern "C" int os_fdtd2d_batch_last_ms(OsFdtd2DBatch *b, float *ms, int64_t *lau
 
 struct OsAdjoint2D {
     OsFdtd2D *h = nullptr;
+    int device = 0;
     int32_t bi0 = 0, bi1 = 0, bj0 = 0, bj1 = 0;
     int32_t n_slots = 0, seg_steps = 0;
     size_t slot_floats = 0;
@@ -3191,6 +3192,7 @@ extern "C" int os_fdtd2d_adjoint_create(OsFdtd2D *h, int32_t box_i0, int32_t box
     OS_CHECK(n_slots >= 1 && segment_steps >= 1, OS_ERR_INVALID, "os_fdtd2d_adjoint_create: bad checkpoint layout");
     std::unique_ptr<OsAdjoint2D> a(new OsAdjoint2D());
     a->h = h;
+    a->device = h->device;
     a->bi0 = box_i0;
     a->bi1 = box_i1;
     a->bj0 = box_j0;
@@ -3226,10 +3228,12 @@ extern "C" int os_fdtd2d_adjoint_create(OsFdtd2D *h, int32_t box_i0, int32_t box
 
 extern "C" int os_fdtd2d_adjoint_destroy(OsAdjoint2D *a) {
     if (!a) return OS_OK;
-    cudaSetDevice(a->h->device);
-    cudaStreamSynchronize(a->h->stream);
+    // the engine may be gone already (a collector takes the two in any order); its recordings end at ev_rec, and freeing the
+    // arrays waits for the device
+    cudaSetDevice(a->device);
     if (a->adj_stream) cudaStreamSynchronize(a->adj_stream);
     for (int b = 0; b < 2; ++b) {
+        if (a->ev_rec[b]) cudaEventSynchronize(a->ev_rec[b]);
         for (cudaGraphExec_t g : a->rec_graph[b])
             if (g) cudaGraphExecDestroy(g);
         for (cudaGraphExec_t g : a->sweep_graph[b])

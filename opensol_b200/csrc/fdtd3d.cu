@@ -211,7 +211,8 @@ static Em3DBox fused_box(const OsFdtd3D *h) {
 }
 
 // variant 3's lean kernel: rows of a multiple of 8 cells (16-byte vectors; the 16-bit id rows are a multiple of 16 bytes, as
-// a tensor map's stride must be), boxes no larger than the grid (the id box is 144 cells wide, the tallest 17 rows), z CPML rows that fit one byte.
+// a tensor map's stride must be), boxes no larger than the grid (the id box is 144 cells wide, the tallest 17 rows), z CPML
+// rows that fit one byte.
 static bool lean_ok(const OsFdtd3D *h) {
     return h->grid.nz % 8 == 0 && h->grid.nz >= Em3DLeanLayout<16>::WM && h->grid.ny >= 17 &&
            h->cpml[2].nr <= EM3D_LEAN_MAX_ZROWS;

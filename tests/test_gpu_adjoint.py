@@ -154,6 +154,23 @@ def test_a_recomputation_that_gave_up_is_reported():
     adj.close()
 
 
+def test_an_engine_closed_before_its_adjoint():
+    """The adjoint's handle can be closed after its engine's (a collector takes the two in any order)."""
+    eps = _eps_box()
+    sim, mon = _product(eps)
+    adj = FluxAdjoint2D(sim, mon, 0, BOX, 100, checkpoint_every=50)
+    adj.forward(eps)
+    g = adj.backward()
+    adj.forward(eps)
+    sim.em.engine.close()
+    adj.close()
+    sim, mon = _product(eps)
+    adj = FluxAdjoint2D(sim, mon, 0, BOX, 100, checkpoint_every=50)
+    adj.forward(eps)
+    np.testing.assert_array_equal(adj.backward(), g)
+    adj.close()
+
+
 def test_torch_autograd_function():
     import torch
     eps = _eps_box()
