@@ -3115,7 +3115,7 @@ struct OsAdjoint2D {
     Ez2DParams rec_params[2][2];
     const float *rec_values[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
     cudaGraphExec_t sweep_graph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};   // per rec buffer and parity
-    int sweep_monitor[2][2] = {{-1, -1}, {-1, -1}};
+    Ez2DAdjParams sweep_params[2][2];   // and the arguments each was captured with
     int64_t graph_launches = 0;
 };
 
@@ -3408,13 +3408,15 @@ extern "C" int os_fdtd2d_adjoint_segment(OsAdjoint2D *a, int32_t slot, int64_t s
         OS_CUDA(cudaStreamSynchronize(as));   // the host rows above are released on return
     }
     const int par = a->e_par;
+    Ez2DAdjParams common = adj_params(a);   // the arguments of every step
+    common.line_normal = mon.normal_axis, common.line_position = mon.position;
+    common.line_lo = mon.lo, common.line_n = n_line;
+    common.row_of_step = a->src_row.ptr, common.de_rows = a->src_e.ptr, common.dh_rows = a->src_h.ptr;
     auto sweep = [&](int32_t steps) -> int {
-        Ez2DAdjParams q = adj_params(a);
+        Ez2DAdjParams q = common;
         const dim3 ablock(32, 8);
         const dim3 agrid((unsigned)((h->grid.ny + 31) / 32), (unsigned)((h->grid.nx + 7) / 8));
         const float *rec = a->rec[rb].ptr;
-        q.line_normal = mon.normal_axis, q.line_position = mon.position, q.line_lo = mon.lo, q.line_n = n_line;
-        q.row_of_step = a->src_row.ptr, q.de_rows = a->src_e.ptr, q.dh_rows = a->src_h.ptr;
         int e = par;
         for (int32_t k = steps - 1; k >= 0; --k) {
             if (k == steps - 1) {   // later steps' sources are added by the H kernel of the step after them
@@ -3450,11 +3452,11 @@ extern "C" int os_fdtd2d_adjoint_segment(OsAdjoint2D *a, int32_t slot, int64_t s
     };
     if (n_steps == a->seg_steps) {
         cudaGraphExec_t &exec = a->sweep_graph[rb][par];
-        if (exec && a->sweep_monitor[rb][par] != monitor_id) {
+        if (exec && memcmp(&common, &a->sweep_params[rb][par], sizeof common)) {
             OS_CUDA(cudaGraphExecDestroy(exec));
             exec = nullptr;
         }
-        a->sweep_monitor[rb][par] = monitor_id;
+        memcpy(&a->sweep_params[rb][par], &common, sizeof common);
         OS_TRY(run_captured(as, exec, [&] { return sweep(n_steps); }));
     } else {
         OS_TRY(sweep(n_steps));

@@ -136,6 +136,35 @@ def test_a_box_or_a_pole_added_later_is_refused(feature):
     adj.close()
 
 
+@pytest.mark.parametrize('variant', [1, 3])
+def test_materials_of_another_kind_between_passes(variant):
+    """Conductivity painted outside the box after a pass: the next gradient is that of a fresh object."""
+    eps = _eps_box()
+
+    def paint(sim):
+        sim.domain.materials.array('sigma_e')[62:66, 20:50] = 2e3
+        sim.domain.materials.version += 1
+        sim.em.materials_changed(('sigma_e',))
+
+    sim, mon = _product(eps)
+    sim.em.engine.configure(variant=variant)
+    adj = FluxAdjoint2D(sim, mon, 0, BOX, N_STEPS, checkpoint_every=64)
+    adj.forward(eps)
+    lossless = adj.backward()
+    paint(sim)
+    J = adj.forward(eps)
+    g = adj.backward()
+    adj.close()
+    sim, mon = _product(eps)
+    paint(sim)
+    sim.em.engine.configure(variant=variant)
+    adj = FluxAdjoint2D(sim, mon, 0, BOX, N_STEPS, checkpoint_every=64)
+    assert adj.forward(eps) == J
+    np.testing.assert_array_equal(adj.backward(), g)
+    assert np.abs(g - lossless).max() > 1e-3 * np.abs(lossless).max()
+    adj.close()
+
+
 def test_a_recomputation_that_gave_up_is_reported():
     """A backward pass whose recomputation left on its bounded wait (the test hook: 1 ms) raises instead of returning a
     gradient; the next pass is clean."""
