@@ -3265,6 +3265,12 @@ extern "C" int os_fdtd2d_adjoint_reset(OsAdjoint2D *a) {
     OS_CHECK(a, OS_ERR_INVALID, "os_fdtd2d_adjoint_reset: null handle");
     OS_TRY(bind_device(a->h));
     cudaStream_t s = a->h->stream;
+    // the zeroing follows every earlier sweep (a backward pass that ended with an error may have left one running), and the
+    // adjoint stream's next sweep the zeroing, by its own wait for its recording on the engine stream
+    for (int b = 0; b < 2; ++b) {
+        if (a->swept_pending[b]) OS_CUDA(cudaStreamWaitEvent(s, a->ev_swept[b], 0));
+        a->swept_pending[b] = false;
+    }
     for (int b = 0; b < 2; ++b) {
         for (DeviceArray<float> *d : {&a->le[b], &a->lhx[b], &a->lhy[b]})
             OS_CUDA(cudaMemsetAsync(d->ptr, 0, d->bytes(), s));
@@ -3275,12 +3281,6 @@ extern "C" int os_fdtd2d_adjoint_reset(OsAdjoint2D *a) {
     }
     OS_CUDA(cudaMemsetAsync(a->grad.ptr, 0, a->grad.bytes(), s));
     a->e_par = 0;
-    // the adjoint stream's next sweep must also follow these zeroings and every earlier sweep: one wait on the engine
-    // stream, which a sweep's own wait for its recording orders anyway; earlier sweeps are joined here
-    for (int b = 0; b < 2; ++b) {
-        if (a->swept_pending[b]) OS_CUDA(cudaStreamWaitEvent(s, a->ev_swept[b], 0));
-        a->swept_pending[b] = false;
-    }
     return OS_OK;
 }
 

@@ -9,6 +9,7 @@ from oracle import adjoint2d
 from oracle.fdtd2d import OracleEz2D
 
 import opensol_b200 as ob
+from opensol_b200 import adjoint as adj_module
 from opensol_b200.adjoint import FluxAdjoint2D, flux_objective
 
 pytestmark = pytest.mark.gpu
@@ -162,6 +163,35 @@ def test_materials_of_another_kind_between_passes(variant):
     assert adj.forward(eps) == J
     np.testing.assert_array_equal(adj.backward(), g)
     assert np.abs(g - lossless).max() > 1e-3 * np.abs(lossless).max()
+    adj.close()
+
+
+def test_a_backward_pass_begun_again():
+    """A backward pass broken off between its segments leaves sweeps running; the next one starts behind them."""
+    eps = _eps_box()
+    sim, mon = _product(eps)
+    adj = FluxAdjoint2D(sim, mon, 0, BOX, N_STEPS, checkpoint_every=64)
+    adj.forward(eps)
+    g = adj.backward()
+    lib = adj_module._native.load()
+
+    class Broken:   # the library whose third segment fails on the host
+        calls = 0
+
+        def __getattr__(self, name):
+            if name == 'os_fdtd2d_adjoint_segment':
+                Broken.calls += 1
+                if Broken.calls == 3:
+                    raise InterruptedError
+            return getattr(lib, name)
+
+    adj.forward(eps)
+    with pytest.MonkeyPatch.context() as patch:
+        patch.setattr(adj_module._native, 'load', lambda: Broken())
+        with pytest.raises(InterruptedError):
+            adj.backward()
+    adj.forward(eps)
+    np.testing.assert_array_equal(adj.backward(), g)
     adj.close()
 
 
