@@ -248,9 +248,11 @@ int os_fdtd2d_advance_noalloc(OsFdtd2D *h, int64_t n_steps, const float *line_va
  * double-buffered kernels, tile_rows rows per interior tile (0, the default: chosen from the grid so that the tiles
  * fill the device's warp slots once, 8..128 rows) and the frame around the interior advanced one step per launch;
  * variant 2 the same with the blocked general kernel on the frame; variant 0 launches one H and one E kernel per
- * step; variant 3 (what the Python engines ask for) is automatic: where the grid fits the chip (1.3 to 2 M cells), a
- * whole chunk of steps runs in one cooperative launch with the fields in registers, whatever sources, poles, plane-wave
- * boxes, maps and probes the engine has; elsewhere, under stream capture, with profiling on and in
+ * step; variant 3 (what the Python engines ask for) is automatic: a whole chunk of steps runs in one cooperative launch
+ * with the fields in registers, whatever sources, poles, plane-wave boxes, maps and probes the engine has, where the grid
+ * fits (on 148 multiprocessors 1180 rows of up to 1280 columns, 2360 of 768, about 3000 of 512; fewer with conductivity,
+ * magnetic cells, maps or poles; with a plane-wave box or poles also up to 2560 columns) and the chunk has the few steps
+ * from which that is the quicker form; elsewhere, under stream capture, with profiling on and in
  * os_fdtd2d_advance_noalloc, variant 1 runs.
  * Every choice gives bit-identical results.  No open_sol counterpart (open_sol launches per half step). */
 int os_fdtd2d_configure(OsFdtd2D *h, int32_t variant, int32_t steps_per_launch, int32_t tile_rows);

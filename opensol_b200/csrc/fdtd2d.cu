@@ -1930,7 +1930,7 @@ static int resident_max_rows(const OsFdtd2D *h, const Res2DJob &job, int columns
 
 // Whether a chunk of n_steps of the handle runs in the resident form now (job, shape and smem filled), planning its strips
 // on the first call.  It takes every feature of the per-step kernels within the parameter block's limits, on any grid whose
-// strips fit a kernel shape (registers: 1.3 to 2 M cells) and a multiprocessor's shared memory; stream capture keeps the
+// strips fit a kernel shape (registers) and a multiprocessor's shared memory; stream capture keeps the
 // launch-per-step forms, whose work a captured graph may replay beside other kernels.
 static int resident_applies(OsFdtd2D *h, int64_t n_steps, Res2DJob &job, int *shape, size_t *smem, bool *yes) {
     *yes = false;
@@ -3040,9 +3040,10 @@ extern "C" int os_fdtd2d_batch_advance(OsFdtd2DBatch *b, OsFdtd2D *const *handle
     OS_CUDA(cudaSetDevice(b->device));
     OS_CUDA(cudaEventRecord(b->ev_start, b->stream));
     // When every job's grid fits the chip, each runs its chunk alone, one after another, in one resident launch:
-    // measured on streams of whole jobs, 16 of 286-930 cells a side took 157 ms against 215 in shared blocked launches,
-    // 48 of 286-542 490 against 600.  With a larger job among them all share the blocked launches, which its tiles
-    // keep busy anyway (32 jobs of 286-2078: 1340 ms together, 1390 with the small ones apart).
+    // measured on streams of whole jobs (fastest of six passes; device time in brackets), 16 of 286-930 cells a side took
+    // 149 ms (103) against 204 (170) in shared blocked launches, 8 of 286-630 46 (27) against 72 (58), 48 of 286-542 435 (387)
+    // against 528 (521), 48 of 230-330 314 (269) against 370 (312).  With a larger job among them all share the blocked
+    // launches, which its tiles keep busy.
     struct Resident {
         Res2DJob job{};
         int shape = -1;

@@ -17,10 +17,11 @@
 // multiply into a packed add.  Sources, plane-wave boxes, poles, probes, field maps and the flux lines' samples are
 // handled inside the step; the flux lines' running sums are folded once per chunk from the staged samples.
 //
-// What bounds it: small strips (240 x 120 cells) wait for the mail, about 1 us from store to poll across L2, plus two
-// block barriers; large ones (1075 x 1075) the issue rate of the row updates.  Measured on a B200, device time per step
-// against the launches per step before it: 270 x 120 cells 2.0 us (15), 441 x 393 lossy 3.6 us (20), 1075 x 1075 6.1 us
-// (17), 930 x 730 H_z 4.9 us (18).  Fields in shared memory instead of registers (one cell at a time) took 18 us at
+// What bounds it: small strips (270 x 120 cells) wait for the mail, about 1 us from store to poll across L2, plus two
+// block barriers (6.6 % of the issue slots used); large ones (1075 x 1075) the latency of the row updates at the 17 warps a
+// multiprocessor that the registers leave (80 instructions per row of two columns and phase, 44 % of the issue slots, a fifth
+// of a warp's time at the barriers).  Measured on a B200, device time per step against the launches per step before it: 270 x
+// 120 cells 2.2 us (15), 441 x 393 lossy 3.6 us (20), 1075 x 1075 5.7 us (17), 930 x 730 H_z 5.2 us (18).  Fields in shared memory instead of registers (one cell at a time) took 18 us at
 // 1075 x 1075; so did polling one mailed word after the other (an L2 round trip each).
 //
 // GEN adds what plain lossless runs do not need: ca / da / db words, field maps, poles, plane-wave boxes.
@@ -192,7 +193,7 @@ extern __shared__ __align__(16) unsigned char res_smem[];   // the block's share
 
 // Plane-wave boxes: each box's incident line in shared memory is four arrays of aux_n floats at `at`: E cells, H cells
 // and their coefficients.  The corrections of the boxes' x sides on a thread's columns j0 .. j0 + C - 1 of row i (the y
-// sides are ResStrip::tfsf_columns'): `v` is H_y after the H update or E_z after the E update of an E_z engine, H_z after
+// sides are ResStrip::tfsf_ab's): `v` is H_y after the H update or E_z after the E update of an E_z engine, H_z after
 // its update or E_y after the E update of an H_z engine.
 template <int C>
 static __device__ __noinline__ float4 res_tfsf_row(const Res2DJob &p, int at, bool e_phase, int i, int j0, float4 in) {
@@ -1342,11 +1343,11 @@ __global__ void __launch_bounds__(NT, 1) res2d_kernel(const __grid_constant__ Re
 // The kernels' shapes: C columns a thread, up to RT rows a strip, up to NT threads, in order of preference (fewest
 // registers first).  The register file bounds them: NT threads have 65,536 / NT registers each (in steps of 128
 // threads: 96 at 640, 128 at 512, 168 at 384, 255 at 256), of which 3 C RT hold fields and about 45 the rest.
-// Four columns a thread run at about half the rate of two (fewer warps, spills): little or nothing faster than the
-// blocked kernels, so only runs that those do not take (poles, plane-wave boxes: about 50 us a step in launches per
-// half step) use the shape.  Measured, us per step here and blocked, E_z / H_z: 1110 x 1130 7.2, 15.6 / 8.4, 18.9; 530 x
-// 1980 9.1, 13.0 / 12.6, 12.9; 830 x 1430 12.6, 14.4 / 15.1, 17.8; 3430 x 330 14.1, 15.2 / 14.0, 16.9; with four columns
-// and 8 to 16 rows 1130 x 1430 15.3, 14.4 and 1730 x 980 18.1, 13.0.
+// Four columns a thread run at about half the rate of two (fewer warps, spills).  Runs that the blocked kernels do not take
+// (poles, plane-wave boxes: 30 to 60 us a step in launches per half step) use them; runs that those take do not.  With an
+// earlier build's plain four-column kernels, us per step resident and blocked, E_z / H_z: up to 6 rows 530 x 1980 9.1, 13.0 /
+// 12.6, 12.9 and 830 x 1430 12.6, 14.4 / 15.1, 17.8, from 8 rows 1130 x 1430 15.3, 14.4 and 1730 x 980 18.1, 13.0: a gain of up
+// to 1.4 on strips of a few wide rows is left.
 struct ResShape {
     int c, rt, nt;
     bool blocked_is_faster;

@@ -221,8 +221,9 @@ class FDTDEngine2D_Ez:
         advancing steps_per_launch (1..4, default 3) steps per launch with tile_rows rows per interior tile (0, the
         default: chosen from the grid), the frame one step per launch; variant 2 = the same with the blocked general
         kernel on the frame; variant 0 = one H and one E kernel per step; variant 3 (a new engine's choice) = the whole
-        chunk in one launch with the fields in shared memory where the grid fits the chip, else variant 1.  Asking for
-        steps_per_launch or tile_rows alone picks the blocked kernels they belong to."""
+        chunk in one launch with the fields in registers where the grid fits the chip and the chunk is long enough for
+        that to pay, else variant 1.  Asking for steps_per_launch or tile_rows alone picks the blocked kernels they
+        belong to."""
         if variant is not None:
             self.variant = int(variant)
         elif self.variant == 3 and (steps_per_launch is not None or tile_rows is not None):
@@ -267,7 +268,9 @@ class FDTDEngine2D_Ez:
 
     def set_stall_probe(self, wait_ns):
         """Test hook of the bounded waits (0: off): one warp of the next blocked advances waits on a barrier nothing
-        completes, at most wait_ns ns, and gives up; the next synchronising call raises RuntimeError."""
+        completes, at most wait_ns ns, and gives up; the first strip of the next resident launches (an adjoint's
+        recomputations among them) sends nothing for wait_ns ns and leaves.  The next synchronising call raises
+        RuntimeError."""
         _native.check(_native.load().os_fdtd2d_set_stall_probe(self.handle, int(wait_ns)))
 
     def kernel_times(self):
@@ -468,10 +471,11 @@ class FDTDEngine2D_Hz(FDTDEngine2D_Ez):
     def configure(self, variant=None, steps_per_launch=None, tile_rows=None):
         """variant 1: interior + border kernel per step, tile_rows interior rows per CTA (0 = chosen per grid); variant
         0: one H_z and one E kernel per step; variant 3 (a new engine's choice): the whole chunk in one launch with the
-        fields in shared memory where the grid fits the chip, else variant 1.  steps_per_launch 2 (default) or 1: with 2, where the grid
-        has no conductivity, no magnetic cells and rows of a multiple of 4 cells, the interior box advances two steps
-        per launch (the border two single steps through a scratch field set, made here) except where the next step is
-        a sampled one; a TFSF box or poles keep one step per launch."""
+        fields in registers where the grid fits the chip and the chunk is long enough for that to pay, else variant 1.
+        steps_per_launch 2 (default) or 1: with 2, where the grid has no conductivity, no magnetic cells and rows of a
+        multiple of 4 cells, the interior box advances two steps per launch (the border two single steps through a
+        scratch field set, made here) except where the next step is a sampled one; a TFSF box or poles keep one step
+        per launch."""
         super().configure(variant, steps_per_launch, tile_rows)
 
     def autotune(self, candidates=None, repeats=4):

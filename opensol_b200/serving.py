@@ -134,7 +134,9 @@ def make_job_specs(n_jobs=256, rate=20.0, seed=7, side_range=(256, 2048), steps_
 
 
 def build_job(spec, device=0, steps_per_launch=3, tile_rows=0):
-    """(Simulation, flux monitors) of a request, finalized and on the device."""
+    """(Simulation, flux monitors) of a request, finalized and on the device.  steps_per_launch 3 with tile_rows 0 leaves
+    the kernels to the engine (resident launches where the grid fits the chip, else three steps per blocked launch);
+    other values pick the blocked kernels (so does configure(variant=1) on the engine, at three steps)."""
     from .simulation import Simulation
     window = spec.side * spec.dx
     sim = Simulation(window, window, spec.dx, npml=spec.npml, boundaries='pml', verbose=False, device=device)
@@ -177,8 +179,9 @@ class _Active:
 
 
 class ServingLoop:
-    """Admission by memory budget and slots, all active jobs stepped together in batched launches (three steps per
-    blocked launch, as for one job alone).
+    """Admission by memory budget and slots, all active jobs stepped together: in one resident launch per job and tick
+    where every job of the tick fits the chip, else in batched launches (three steps per blocked launch, as for one
+    job alone).  steps_per_launch and tile_rows as in build_job.
 
     A tick advances every active job by chunk_steps, or by what it has left when that is less: the jobs with a full
     chunk left go together in one batched call, and the few that finish inside the tick in one call per remaining
