@@ -1928,6 +1928,21 @@ static int resident_max_rows(const OsFdtd2D *h, const Res2DJob &job, int columns
     return job.da && ny < 300 ? 9 : 17;
 }
 
+// Whether the field maps leave the resident form quicker.  A thread adds the terms of its cells one after the other, 0.4 to 0.6
+// us each, where the blocked kernels have a launch of its own over the map, 3.5 us per million terms: the line is a number of
+// terms a thread and step, lower the taller the strip.  Measured, us per step here and in the blocked kernels: E_z 3 rows 15
+// terms 13, 15; 8 rows 10 terms 12.5, 17, 39 terms 28.5, 24.6; 14 rows 4 terms 11.3, 12.2, 17 terms 15.0, 14.0; H_z 3 rows 11
+// terms 10, 16, 44 terms 27.8, 18.5; 8 rows 2 terms 12.8, 13.1, 7 terms 15.3, 14.5, 118 terms 82.7, 39.9; 14 rows 0.4 terms
+// 12.6, 16.9, 3 terms 13.2, 12.9, 207 terms 99.5, 32.7.  Launches per half step leave room for 15 terms more.
+static bool resident_maps_pay(const OsFdtd2D *h, int rows, int columns, bool blocked) {
+    double terms = 0.0;
+    for (auto &d : h->maps)
+        terms += (double)std::min((rows + d->ds - 1) / d->ds, d->mx) * std::min((columns + d->ds - 1) / d->ds, d->my) * d->nf;
+    terms *= (h->polarization == 1 ? 3.0 : 1.0) / (double)h->sample_interval;
+    const double room = (h->polarization == 1 ? 26.0 - 2.9 * rows : 22.0 - 1.1 * rows) + (blocked ? 0.0 : 15.0);
+    return terms <= std::max(room, 0.75);
+}
+
 // Whether a chunk of n_steps of the handle runs in the resident form now (job, shape and smem filled), planning its strips
 // on the first call.  It takes every feature of the per-step kernels within the parameter block's limits, on any grid whose
 // strips fit a kernel shape (registers) and a multiprocessor's shared memory; stream capture keeps the
@@ -1959,7 +1974,8 @@ static int resident_applies(OsFdtd2D *h, int64_t n_steps, Res2DJob &job, int *sh
     if (*shape < 0) return OS_OK;
     job = resident_job(h);
     if (n_steps < resident_min_steps(h, max_rows, blocked, res2d_general(job)) ||
-        max_rows > resident_max_rows(h, job, res2d_columns(*shape)))
+        max_rows > resident_max_rows(h, job, res2d_columns(*shape)) ||
+        !resident_maps_pay(h, max_rows, res2d_columns(*shape), blocked))
         return OS_OK;
     const bool lo = g.cpml_sides & 1, hi = g.cpml_sides & 2;
     auto rows_in = [](int a, int b, int c, int d) { return std::max(0, std::min(b, d) - std::max(a, c)); };

@@ -132,7 +132,7 @@ SHAPES = {
     (2, 8, 640): [dict(nx=1100, ny=1131, boundaries='pml'), dict(nx=700, ny=1050, boundaries='periodic_y', lossy=True),
                   dict(nx=1020, ny=1203, boundaries='periodic_x', maps=(7,), probes=2)],
     (2, 16, 384): [dict(nx=2300, ny=301, boundaries='pml', probes=3), dict(nx=1330, ny=90, boundaries='periodic', lossy=True),
-                   dict(nx=1900, ny=203, boundaries='periodic_y', maps=(5,)), dict(nx=1500, ny=77, boundaries='pml', tfsf=2,
+                   dict(nx=1900, ny=203, boundaries='periodic_y', maps=(30,)), dict(nx=1500, ny=77, boundaries='pml', tfsf=2,
                                                                                    lines=())],
     (2, 24, 256): [dict(nx=2900, ny=121, boundaries='pml'), dict(nx=2700, ny=63, boundaries='periodic_y', probes=1),
                    dict(nx=2800, ny=130, boundaries='pml', tfsf=1, lines=())],
@@ -188,7 +188,7 @@ def test_short_chunks_take_the_quicker_form(pol, rows, ez_steps, hz_steps, featu
 # polarisation, features, rows a strip up to which they run resident, columns
 TALL = [('ez', {}, 20, 64), ('hz', {}, 22, 64), ('hz', dict(lossy=True), 5, 1040), ('ez', dict(tfsf=1, lines=()), 12, 60),
         ('hz', dict(lossy=True), 9, 60), ('ez', dict(lossy=True), 17, 60), ('hz', dict(magnetic=True), 9, 60),
-        ('ez', dict(magnetic=True), 9, 60), ('ez', dict(magnetic=True), 17, 302), ('hz', dict(maps=(3,)), 16, 60),
+        ('ez', dict(magnetic=True), 9, 60), ('ez', dict(magnetic=True), 17, 302), ('hz', dict(maps=(40,)), 16, 60),
         ('ez', dict(maps=(3,)), 17, 60), ('ez', dict(poles=(DRUDE,)), 14, 60), ('hz', dict(poles=(DRUDE,)), 12, 60),
         ('ez', dict(poles=(LORENTZ,)), 12, 820), ('hz', dict(poles=(LORENTZ,)), 8, 1340)]
 
@@ -198,6 +198,17 @@ def test_tall_strips_take_the_quicker_form(pol, features, rows, ny):
     for r in (rows, rows + 1):
         args = dict(pol=pol, nx=148 * r - 12 - 2 * r, ny=ny - 12, boundaries='pml', npml=6, seed=r, **features)
         _compare(args, (45, 2 * rows + 2), resident=[r == rows] * 2)
+
+
+@pytest.mark.parametrize('pol, rows, maps, resident', [
+    ('ez', 8, (1, 1, 1), True), ('ez', 8, (1, 1, 1, 1), False), ('ez', 3, (1, 1, 1, 1), True), ('ez', 14, (1,), True),
+    ('ez', 14, (1, 1), False), ('hz', 3, (1, 1, 1, 1), True), ('hz', 4, (1, 1, 1, 1), False), ('hz', 8, (2,), True),
+    ('hz', 8, (1,), False), ('hz', 12, (9,), False), ('hz', 12, (13,), True)])
+def test_maps_with_many_terms_take_the_quicker_form(pol, rows, maps, resident):
+    args = dict(pol=pol, nx=148 * rows - 12 - 2 * rows, ny=48, boundaries='pml', npml=6, seed=rows, maps=maps)
+    sim, _out = _sim(**args)
+    assert sim.em.engine.sample_interval == 9   # two frequencies a map: 2 x 2 x rows / 9 terms a thread and step, H_z 3 times
+    _compare(args, (40, 31), resident=[resident] * 2)
 
 
 def test_resident_chunk_past_the_staged_samples():
