@@ -3055,11 +3055,11 @@ extern "C" int os_fdtd2d_batch_advance(OsFdtd2DBatch *b, OsFdtd2D *const *handle
     }
     OS_CUDA(cudaSetDevice(b->device));
     OS_CUDA(cudaEventRecord(b->ev_start, b->stream));
-    // When every job's grid fits the chip, each runs its chunk alone, one after another, in one resident launch:
-    // measured on streams of whole jobs (fastest of six passes; device time in brackets), 16 of 286-930 cells a side took
-    // 149 ms (103) against 204 (170) in shared blocked launches, 8 of 286-630 46 (27) against 72 (58), 48 of 286-542 435 (387)
-    // against 528 (521), 48 of 230-330 314 (269) against 370 (312).  With a larger job among them all share the blocked
-    // launches, which its tiles keep busy.
+    // When every job's grid fits the chip, each may run its chunk alone, one after another, in one resident launch; or all
+    // share the blocked launches (as they do with a larger job among them).  Device time, us: a resident job 20 and 3 a row
+    // of its strips, and per step 2.0 and 3.4 per million cells; the shared launches per step 10, 0.9 a job and 7.7 per
+    // million cells of all (fitted to ticks of 8 to 512 steps).  Measured per step, resident and shared, 512-step ticks: 3 jobs of 330 cells a
+    // side 8, 15; 8 of 830-1030 40, 67; 16 of 286-930 57, 67; 48 of 286-542 138, 117; 48 of 130-190 107, 63.
     struct Resident {
         Res2DJob job{};
         int shape = -1;
@@ -3067,9 +3067,15 @@ extern "C" int os_fdtd2d_batch_advance(OsFdtd2DBatch *b, OsFdtd2D *const *handle
     };
     std::vector<Resident> runs((size_t)n_jobs);
     bool all = true;
-    for (int32_t q = 0; q < n_jobs && all; ++q)
-        OS_TRY(resident_applies(handles[q], n_steps, runs[q].job, &runs[q].shape, &runs[q].smem, &all));
-    if (!all) {
+    double in_turn = 0.0, shared = (double)n_steps * (10.0 + 0.9 * n_jobs);
+    for (int32_t q = 0; q < n_jobs && all; ++q) {
+        OsFdtd2D *h = handles[q];
+        OS_TRY(resident_applies(h, n_steps, runs[q].job, &runs[q].shape, &runs[q].smem, &all));
+        const double mcells = 1e-6 * (double)cells(h);
+        in_turn += 20.0 + 3.0 * (h->grid.nx / h->sm_count + 1) + (double)n_steps * (2.0 + 3.4 * mcells);
+        shared += (double)n_steps * 7.7 * mcells;
+    }
+    if (!all || in_turn > shared) {
         OS_TRY(batch_advance_blocked(b, handles, n_jobs, n_steps, line_values, first_samples, n_samples, phases));
     } else {
         for (int32_t q = 0; q < n_jobs; ++q) {

@@ -180,7 +180,7 @@ class _Active:
 
 class ServingLoop:
     """Admission by memory budget and slots, all active jobs stepped together: in one resident launch per job and tick
-    where every job of the tick fits the chip, else in batched launches (three steps per blocked launch, as for one
+    where every job of the tick fits the chip and the jobs are few, else in batched launches (three steps per blocked launch, as for one
     job alone).  steps_per_launch and tile_rows as in build_job.
 
     A tick advances every active job by chunk_steps, or by what it has left when that is less: the jobs with a full

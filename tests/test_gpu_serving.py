@@ -58,6 +58,28 @@ def test_batched_fields_equal_single_advance():
     batch.close()
 
 
+@pytest.mark.parametrize('n, resident', [(2, True), (30, False)])
+def test_few_jobs_in_turn_many_together(n, resident):
+    """A tick of jobs that fit the chip: a few run one resident launch each, many small ones share the blocked launches; the
+    fields are those of each job alone."""
+    specs = _small_specs(n=n, seed=6)
+    batch = serving.BatchAdvancer()
+    sims = [serving.build_job(s)[0] for s in specs]
+    for sim in sims:
+        batch.adopt(sim.em.engine)
+    for steps in (64, 65):
+        batch.advance([sim.em.engine for sim in sims], steps)
+        launches = batch.last_ms()[1]
+        assert launches == 3 * n if resident else launches >= 2 * (steps // 3)   # a launch, two flux folds a job
+    for spec, sim in zip(specs, sims):
+        ref, _ = serving.build_job(spec)
+        ref.em.engine.configure(variant=0)
+        ref.em.engine.advance(129)
+        for name in ('ez', 'hx', 'hy'):
+            np.testing.assert_array_equal(sim.em.engine.read_field(name), ref.em.engine.read_field(name))
+    batch.close()
+
+
 def test_mix_equals_alone_at_stream_sizes():
     """Ten jobs of the serving stream's own kind at sizes 256-1024 cells a side (+30 CPML cells: row lengths that are
     not multiples of 4 included), 600-1500 steps, served together with at most 6 active at once and 256-step ticks
